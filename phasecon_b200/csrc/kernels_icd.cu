@@ -61,11 +61,10 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z)
 // Surrogate weight rho'(d)/d of the qGGMRF potential
 // |d|^(q-p) ... (derivative per XT_ICD_update.c:92-118; value at d = 0 per
 // :119-128): |d|^(q-2) (q - (q-p) t1 / t3) / (t3 sq), t1 = |d|^(q-p) / sqp,
-// t3 = c + t1. Takes isq = 1 / sq and isqp = 1 / sqp. The weight is
-// evaluated ~28 times per voxel update, so it uses the hardware base-2
-// logarithm / exponential (one logarithm for both powers) and reciprocal:
-// FP32 arithmetic whose rounding the FP64 MAP cost, by which the method's
-// result is measured, does not see.
+// t3 = c + t1. The weight is evaluated ~28 times per voxel update, so it uses
+// the hardware base-2 logarithm / exponential (one logarithm for both powers)
+// and reciprocal: FP32 arithmetic whose rounding the FP64 MAP cost, by which
+// the method's result is measured, does not see.
 __device__ __forceinline__ float lg2_hw(float x)
 {
     float r;
@@ -84,151 +83,212 @@ __device__ __forceinline__ float rcp_hw(float x)
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
     return r;
 }
-__device__ __forceinline__ float qg_weight(float d, float q, float qmp, float isq, float isqp, float c, float b0)
+// N weights times their filter coefficients f (which carry the 1 / sq), side by
+// side and without branches, so that the N chains of about 130 cycles run in
+// each other's shadow. isqp = 1 / sqp; at d = 0 the weight is q / (sq c).
+template <int N>
+__device__ __forceinline__ void qg_coef(const float (&d)[N], const float (&f)[N], float q, float qmp, float isqp,
+                                        float c, float qoc, float (&cf)[N])
 {
-    if (d == 0.0f) return b0;
-    const float l = lg2_hw(fabsf(d));
-    const float t1 = ex2_hw(qmp * l) * isqp;
-    const float rt3 = rcp_hw(c + t1);
-    float r = (q - qmp * t1 * rt3) * rt3 * isq;
-    if (q != 2.0f) r *= ex2_hw((q - 2.0f) * l);
-    return r;
-}
-
-template <int KW>
-struct Rec {
-    uint4 w[KW];
-};
-
-template <int KW>
-__device__ __forceinline__ Rec<KW> load_rec(const uint32_t *p)
-{
-    Rec<KW> r;
-    const uint4 *q = reinterpret_cast<const uint4 *>(p);
+    float l[N];
 #pragma unroll
-    for (int i = 0; i < KW; i++) r.w[i] = __ldg(q + i);
-    return r;
-}
-
-template <int KW>
-__device__ __forceinline__ Rec<KW> load_rec_smem(const uint32_t *p)
-{
-    Rec<KW> r;
-    const uint4 *q = reinterpret_cast<const uint4 *>(p);
+    for (int i = 0; i < N; i++) l[i] = lg2_hw(fabsf(d[i]));
 #pragma unroll
-    for (int i = 0; i < KW; i++) r.w[i] = q[i];
-    return r;
-}
-
-// Copy a column's A records (nwords 32-bit words, a multiple of 4, 16-byte
-// aligned on both sides) into shared memory with one TMA bulk copy, issued by
-// thread 0, that completes on the buffer's mbarrier; the copy lands while the
-// CTA works on the current column.
-__device__ __forceinline__ void stage_records(uint32_t *dst, const uint32_t *src, int nwords,
-                                              unsigned long long *bar)
-{
-    if (threadIdx.x != 0) return;
-    const unsigned b = (unsigned)__cvta_generic_to_shared(bar), d = (unsigned)__cvta_generic_to_shared(dst);
-    const unsigned bytes = 4u * (unsigned)nwords;
-    if (bytes == 0) {  // a frame without views: complete the phase with no transfer
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(b) : "memory");
-        return;
+    for (int i = 0; i < N; i++) {
+        const float t1 = ex2_hw(qmp * l[i]) * isqp;
+        const float rt3 = rcp_hw(c + t1);
+        cf[i] = (q - qmp * (t1 * rt3)) * rt3;
     }
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bytes) : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(d),
-                 "l"(src), "r"(bytes), "r"(b)
+    if (q != 2.0f) {
+#pragma unroll
+        for (int i = 0; i < N; i++) cf[i] *= ex2_hw((q - 2.0f) * l[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < N; i++) cf[i] = f[i] * (d[i] == 0.0f ? qoc : cf[i]);
+}
+
+// The one arrival of a copy's mbarrier phase, and the bytes the phase waits for.
+__device__ __forceinline__ void expect_bytes(unsigned long long *bar, int bytes)
+{
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"((unsigned)__cvta_generic_to_shared(bar)),
+                 "r"(bytes)
                  : "memory");
+}
+// One TMA bulk copy into shared memory (16-byte aligned on both sides, a multiple
+// of 16 bytes), issued by one thread; completes on the mbarrier.
+__device__ __forceinline__ void bulk_copy(void *dst, const void *src, unsigned bytes, unsigned long long *bar)
+{
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(dst)),
+                 "l"(src), "r"(bytes), "r"((unsigned)__cvta_generic_to_shared(bar))
+                 : "memory");
+}
+
+// The voxel values a super-voxel's updates read, by bulk copies into shared
+// memory: three planes of (sv + 2)^2 columns -- the SV and its in-plane
+// neighbours in its frame, then the SV's columns in frames f - 1 and f + 1 at
+// the same places of their planes, so that every neighbour of a column sits at a
+// fixed offset from it. A plane's row is contiguous in x ([y][x][z]); cells
+// outside the image or the frames are left alone (never read). Called by one
+// warp; N_z is a multiple of 4, so every row starts on 16 bytes and is a multiple
+// of 16 bytes long. `more`: bytes of a further copy on the same mbarrier phase.
+// No other CTA of the launch writes these columns (same-colour SVs share no
+// neighbour, and frames f +- 1 are on other colours).
+__device__ __forceinline__ void stage_tile(float *tile, const float *x, const Geom &g, int f, int sx, int sy, int sv,
+                                           int more, unsigned long long *bar)
+{
+    const int lane = threadIdx.x & 31, TW = sv + 2, NX = g.N_x, NY = g.N_y, NZ = g.N_z;
+    const size_t nxy = (size_t)NX * NY;
+    const int j0 = sy * sv, k0 = sx * sv;
+    const int ka = max(k0 - 1, 0), kb = min(k0 + sv + 1, NX), ja = max(j0 - 1, 0), jb = min(j0 + sv + 1, NY);
+    const int ke = min(k0 + sv, NX), je = min(j0 + sv, NY);
+    const int frames = (f > 0) + (f + 1 < g.N_time);
+    if (lane == 0) expect_bytes(bar, 4 * NZ * ((jb - ja) * (kb - ka) + frames * (je - j0) * (ke - k0)) + more);
+    __syncwarp();
+    for (int r = lane; r < TW + 2 * sv; r += 32) {
+        if (r < TW) {
+            const int j = j0 - 1 + r;
+            if (j >= 0 && j < NY)
+                bulk_copy(tile + (r * TW + (ka - k0 + 1)) * NZ, x + ((size_t)f * nxy + (size_t)j * NX + ka) * NZ,
+                          4u * (unsigned)((kb - ka) * NZ), bar);
+        } else {
+            const int p = r - TW < sv ? 1 : 2, row = r - TW - (p - 1) * sv, ff = p == 1 ? f - 1 : f + 1, j = j0 + row;
+            if (ff >= 0 && ff < g.N_time && j < NY)
+                bulk_copy(tile + ((p * TW + row + 1) * TW + 1) * NZ, x + ((size_t)ff * nxy + (size_t)j * NX + k0) * NZ,
+                          4u * (unsigned)((ke - k0) * NZ), bar);
+        }
+    }
+}
+
+__device__ __forceinline__ bool try_parity(unsigned long long *bar, uint32_t parity)
+{
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred P;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, P;\n\t}"
+        : "=r"(ok)
+        : "r"((unsigned)__cvta_generic_to_shared(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
 }
 
 // Bounded wait (about 2 s of clock64) for phase `parity` of mbarrier `bar`;
 // returns false if it ran out.
 __device__ __forceinline__ bool wait_parity_bounded(unsigned long long *bar, uint32_t parity)
 {
-    const unsigned a = (unsigned)__cvta_generic_to_shared(bar);
+    if (try_parity(bar, parity)) return true;  // the usual case: the copy landed a column ago
     const long long t0 = clock64();
-    for (;;) {
-        uint32_t ok;
-        asm volatile(
-            "{\n\t.reg .pred P;\n\t"
-            "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
-            "selp.u32 %0, 1, 0, P;\n\t}"
-            : "=r"(ok)
-            : "r"(a), "r"(parity)
-            : "memory");
-        if (ok) return true;
+    while (!try_parity(bar, parity))
         if (clock64() - t0 > 4000000000LL) return false;
-    }
+    return true;
 }
 
-// Every thread waits for buffer b's copy: the n-th copy into a buffer
-// completes the mbarrier's phase n, so the parity of the wait is the count of
-// earlier waits on that buffer (bit b of `phases`, identical in every thread).
+// Wait for buffer b's copy: the n-th copy into a buffer completes the mbarrier's
+// phase n, so the parity of the wait is the count of earlier copies into that
+// buffer (bit b of `phases`, which every thread keeps whether it waits or not).
 // The wait is bounded; a copy that never lands is counted (the host turns the
 // count into an error) and raises the CTA's abort flag: the caller stops
 // updating and staging after the next barrier, and the kernel waits for the
-// late copy once more before it exits (abort_bar / abort_parity).
+// copies in flight once more before it exits (drain_copies).
 // Returns whether this thread's wait saw the copy land.
-__device__ __forceinline__ bool wait_staged(unsigned long long *bar, uint32_t &phases, int b, unsigned &timeouts,
-                                            int &abort, int &abort_bar, uint32_t &abort_parity)
+__device__ __forceinline__ bool wait_staged(unsigned long long *bar, uint32_t phases, int b, unsigned &timeouts,
+                                            int &abort)
 {
-    const uint32_t parity = (phases >> b) & 1u;
-    const bool ok = wait_parity_bounded(bar, parity);
+    const bool ok = wait_parity_bounded(bar, (phases >> b) & 1u);
     if (!ok) {
         timeouts++;
-        abort = 1;  // every writer stores the same values
-        abort_bar = b;
-        abort_parity = parity;
+        abort = 1;
     }
-    phases ^= 1u << b;
     return ok;
 }
 
-template <int KW>
-__device__ __forceinline__ float rec_val(const Rec<KW> &r, int q)
+// Two FP32 values in one 64-bit register pair: the packed FP32 instructions
+// (fma / mul .f32x2) do two lanes' worth of rounding-identical arithmetic per
+// issue slot.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b)
 {
-    // word 1 + q of the record
-    const int wi = 1 + q;
-    const uint4 &u = r.w[wi >> 2];
-    const uint32_t bits = (wi & 3) == 0 ? u.x : (wi & 3) == 1 ? u.y : (wi & 3) == 2 ? u.z : u.w;
-    return __uint_as_float(bits);
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void unpack2(f32x2 v, float &a, float &b)
+{
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
 }
 
+// VEC consecutive detector rows of one sinogram entry, as packed pairs.
 template <int VEC>
-struct VecF;
-template <>
-struct VecF<4> {
-    using T = float4;
-    __device__ static void get(const T &v, float *o) { o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w; }
+struct Rows {
+    f32x2 p[VEC / 2];
 };
-template <>
-struct VecF<2> {
-    using T = float2;
-    __device__ static void get(const T &v, float *o) { o[0] = v.x; o[1] = v.y; }
-};
-
-// Vector reduction into global memory (red.global.add.v{2,4}.f32, sm_90+).
-__device__ __forceinline__ void red_add(float *p, const float (&d)[4])
+// e and w of one entry, loaded where i < n (else they keep what they hold): one
+// predicate and two predicated loads, where an `if` compiles to a branch. e changes
+// under the sweep (other CTAs' reductions land in L2), so it is read from there;
+// w is constant.
+__device__ __forceinline__ void load_entry(Rows<4> &e, Rows<4> &w, const float *pe, const float *pw, int i, int n)
 {
-    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(d[0]), "f"(d[1]), "f"(d[2]), "f"(d[3])
+    asm volatile(
+        "{\n\t.reg .pred P;\n\tsetp.lt.s32 P, %6, %7;\n\t@P ld.global.cg.v2.b64 {%0, %1}, [%4];\n\t"
+        "@P ld.global.nc.v2.b64 {%2, %3}, [%5];\n\t}"
+        : "+l"(e.p[0]), "+l"(e.p[1]), "+l"(w.p[0]), "+l"(w.p[1])
+        : "l"(pe), "l"(pw), "r"(i), "r"(n)
+        : "memory");
+}
+__device__ __forceinline__ void load_entry(Rows<2> &e, Rows<2> &w, const float *pe, const float *pw, int i, int n)
+{
+    asm volatile(
+        "{\n\t.reg .pred P;\n\tsetp.lt.s32 P, %4, %5;\n\t@P ld.global.cg.b64 %0, [%2];\n\t"
+        "@P ld.global.nc.b64 %1, [%3];\n\t}"
+        : "+l"(e.p[0]), "+l"(w.p[0])
+        : "l"(pe), "l"(pw), "r"(i), "r"(n)
+        : "memory");
+}
+
+// Vector reduction into global memory (red.global.add.v{2,4}.f32, sm_90+) where
+// i < n: one predicated instruction (an `if` compiles to a branch).
+__device__ __forceinline__ void red_add(float *p, const Rows<4> &d, int i, int n)
+{
+    float a, b, c, e;
+    unpack2(d.p[0], a, b);
+    unpack2(d.p[1], c, e);
+    asm volatile(
+        "{\n\t.reg .pred P;\n\tsetp.lt.s32 P, %5, %6;\n\t@P red.global.add.v4.f32 [%0], {%1, %2, %3, %4};\n\t}" ::"l"(p),
+        "f"(a), "f"(b), "f"(c), "f"(e), "r"(i), "r"(n)
+        : "memory");
+}
+__device__ __forceinline__ void red_add(float *p, const Rows<2> &d, int i, int n)
+{
+    float a, b;
+    unpack2(d.p[0], a, b);
+    asm volatile("{\n\t.reg .pred P;\n\tsetp.lt.s32 P, %3, %4;\n\t@P red.global.add.v2.f32 [%0], {%1, %2};\n\t}" ::"l"(p),
+                 "f"(a), "f"(b), "r"(i), "r"(n)
                  : "memory");
 }
-__device__ __forceinline__ void red_add(float *p, const float (&d)[2])
-{
-    asm volatile("red.global.add.v2.f32 [%0], {%1, %2};" ::"l"(p), "f"(d[0]), "f"(d[1]) : "memory");
-}
-
 
 struct IcdSmem {
     unsigned long long stage_bar[2];  // completion of the two record buffers' bulk copies
-    float num[kMaxWarps][32], den[kMaxWarps][32];
-    float th1[kMaxWarps][32], th2[kMaxWarps][32];
-    int pos[kMaxWarps][32];
-    float dx[32];
-    int order[kMaxSvCols];
+    float2 nd[kMaxWarps][32];         // per warp and slice: the prior's (num, den)
+    float2 th[kMaxWarps][32];         // per warp and detector row: (theta1, theta2)
+    unsigned pos[kMaxWarps];          // per warp: slices with a positive neighbour, as bits
+    __align__(16) float dx[32];       // per detector row of the chunk: the change of its slice
+    int2 order[kMaxSvCols];           // columns to visit: (index in the image, tile cell << 10 | sources inside the object)
     int ncols, item;
     int abort;              // a record copy did not land in time: stop updating
-    int abort_bar;          // the buffer whose copy was late, and the wait's parity
-    uint32_t abort_parity;
+    unsigned issued[2];     // copies started into each buffer
 };
 
 struct IcdCount {
@@ -261,107 +321,131 @@ __device__ __forceinline__ void flush_counts(IcdCount &cnt, IcdStats *stats)
     cnt.phases = phases;
 }
 
-// theta1 / theta2 partial sums of one lane (VEC detector rows starting at
-// sinogram row offset `row0` within each A entry's row, views gfirst,
-// gfirst + gstride, ... of the column): theta1 = -sum a w e,
-// theta2 = sum a^2 w with a = A value x delta_t (XT_VoxUpdate.c:56-85).
-template <int KW, int kUnroll, int VEC, bool kStaged, int kHuber>
-__device__ __forceinline__ void theta_pass(const IcdConst &K, const uint32_t *col_rec, const float *__restrict__ err,
-                                           const float *__restrict__ wgt, int gfirst, int gstride, int nv, int RW,
-                                           int NT, int row0, float (&th1)[VEC], float (&th2)[VEC])
+// Entry lists. A column's A records (header + values) are unpacked once into a
+// list per view group of (sinogram offset, -a) pairs, a = A value x delta_t: the
+// theta and apply passes then run over exactly the entries there are (2.27 a view
+// at voxel scale 1, of the 3 slots of a record) without decoding or branching.
+// A group's list: slot 0 holds its count and the largest count of the warp's
+// groups, slots 1.. the entries, filled up with entries of weight zero to the
+// multiple (at least one) of the batch that covers that largest count. `cap` slots a group, odd,
+// so that the groups of a warp read different banks.
+__host__ __device__ inline int icd_lanes_per_row(int N_t, int vec)  // lanes over a full chunk's rows, a power of two
 {
-    using VT = typename VecF<VEC>::T;
-    for (int v0 = gfirst; v0 < nv; v0 += kUnroll * gstride) {
-        Rec<KW> R[kUnroll];
-#pragma unroll
-        for (int u = 0; u < kUnroll; u++) {
-            const int v = v0 + u * gstride;
-            if (v < nv) R[u] = kStaged ? load_rec_smem<KW>(col_rec + (size_t)v * RW) : load_rec<KW>(col_rec + (size_t)v * RW);
-            else R[u].w[0].x = 0u;
-        }
-#pragma unroll
-        for (int u = 0; u < kUnroll; u++) {
-            const uint32_t hdr = R[u].w[0].x;
-            const int cnt_q = hdr >> 24;
-            // sinogram rows stay below 2^24 and N_t rows each: 32-bit offsets
-            const unsigned sb = (hdr & 0xFFFFFFu) * (unsigned)NT + (unsigned)row0;
-#pragma unroll
-            for (int q = 0; q < 4 * KW - 1; q++) {
-                if (q < cnt_q) {
-                    float ev[VEC], wv[VEC];
-                    VecF<VEC>::get(__ldcg(reinterpret_cast<const VT *>(err + (sb + (unsigned)(q * NT)))), ev);
-                    VecF<VEC>::get(__ldg(reinterpret_cast<const VT *>(wgt + (sb + (unsigned)(q * NT)))), wv);
-                    const float a = rec_val<KW>(R[u], q) * K.dt;
-#pragma unroll
-                    for (int i = 0; i < VEC; i++) {
-                        float ww = wv[i];
-                        if (kHuber == 1 || (kHuber == 2 && K.huber)) {
-                            const float sw = sqrtf(ww);
-                            if (!(fabsf(ev[i] * sw) < K.huber_T)) ww = K.huber_T * K.huber_delta * sw / fabsf(ev[i]);
-                        }
-                        const float aw = a * ww;
-                        th2[i] += a * aw;
-                        th1[i] -= ev[i] * aw;
-                    }
-                }
-            }
-        }
-    }
+    const int lpr = (N_t < 32 ? N_t : 32) / vec;
+    int p = 1;
+    while (p < lpr) p <<= 1;
+    return p;
+}
+__host__ __device__ inline int icd_list_cap(int views_per_group, int kmax, int batch)
+{
+    return (1 + (views_per_group * kmax + batch - 1) / batch * batch) | 1;
 }
 
-// One column's theta: every lane's partial sums (theta_pass, when `run`),
-// folded over the view groups of the warp and stored by group 0 into the
-// warp's row of S.th1 / S.th2.
-template <int KW, int kUnroll, int VEC, bool kStaged, int kHuber>
-__device__ __forceinline__ void theta_column(const IcdConst &K, const uint32_t *col_rec, const float *__restrict__ err,
-                                             const float *__restrict__ wgt, int gfirst, int gstride, int nv, int RW,
-                                             int NT, int row0, bool run, int lprp, int grp, int t0, int warp,
-                                             IcdSmem &S)
+// Unpack the records of view group `group` (views group, group + gstride, ...
+// from v_begin below v_end) into `list`; called by all lanes of a warp, lane tq of
+// the group's lprp lanes taking every lprp-th of its views.
+// where i < n
+__device__ __forceinline__ void put_entry(uint2 *p, unsigned off, float na, int i, int n)
 {
-    float th1[VEC], th2[VEC];
-#pragma unroll
-    for (int i = 0; i < VEC; i++) th1[i] = th2[i] = 0.0f;
-    if (run) theta_pass<KW, kUnroll, VEC, kStaged, kHuber>(K, col_rec, err, wgt, gfirst, gstride, nv, RW, NT, row0, th1, th2);
-    for (int off = lprp; off < 32; off <<= 1) {
-#pragma unroll
-        for (int i = 0; i < VEC; i++) {
-            th1[i] += __shfl_xor_sync(0xffffffffu, th1[i], off);
-            th2[i] += __shfl_xor_sync(0xffffffffu, th2[i], off);
+    asm volatile("{\n\t.reg .pred P;\n\tsetp.lt.s32 P, %3, %4;\n\t@P st.shared.v2.b32 [%0], {%1, %2};\n\t}" ::"r"(
+                     (unsigned)__cvta_generic_to_shared(p)),
+                 "r"(off), "r"(__float_as_uint(na)), "r"(i), "r"(n)
+                 : "memory");
+}
+
+template <int kBatch>
+__device__ __forceinline__ void unpack_records(const uint32_t *rec, int RW, int NT, float dt, uint2 *list, int group,
+                                               int gstride, int v_begin, int v_end, int tq, int lprp)
+{
+    int total = 0;
+    for (int base = v_begin; base < v_end; base += gstride * lprp) {  // uniform over the CTA
+        const int v = base + group + tq * gstride;
+        const uint32_t *r = rec + (size_t)v * RW;
+        uint4 head = make_uint4(0u, 0u, 0u, 0u);  // header and the first three values
+        if (v < v_end) head = *reinterpret_cast<const uint4 *>(r);
+        const int n = (int)(head.x >> 24);
+        int incl = n;
+        for (int o = 1; o < lprp; o <<= 1) {
+            const int up = __shfl_up_sync(0xffffffffu, incl, o, lprp);
+            if (tq >= o) incl += up;
         }
+        uint2 *dst = list + 1 + total + incl - n;
+        // sinogram rows stay below 2^24 and N_t rows each: 32-bit offsets
+        const unsigned off = (head.x & 0xFFFFFFu) * (unsigned)NT;
+        put_entry(dst, off, -(__uint_as_float(head.y) * dt), 0, n);
+        put_entry(dst + 1, off + (unsigned)NT, -(__uint_as_float(head.z) * dt), 1, n);
+        put_entry(dst + 2, off + 2u * (unsigned)NT, -(__uint_as_float(head.w) * dt), 2, n);
+        for (int q = 3; q < n; q++)
+            dst[q] = make_uint2(off + (unsigned)(q * NT), __float_as_uint(-(__uint_as_float(r[1 + q]) * dt)));
+        total += __shfl_sync(0xffffffffu, incl, lprp - 1, lprp);
     }
-    if (grp == 0 && run) {
-#pragma unroll
-        for (int i = 0; i < VEC; i++) {
-            S.th1[warp][t0 + i] = th1[i];
-            S.th2[warp][t0 + i] = th2[i];
-        }
-    }
+    const int most = __reduce_max_sync(0xffffffffu, total);
+    const int padded = max(1, (most + kBatch - 1) / kBatch) * kBatch;
+    for (int i = total + tq; i < padded; i += lprp) list[1 + i] = make_uint2(0u, 0u);
+    if (tq == 0) list[0] = make_uint2((unsigned)total, (unsigned)most);
+}
+
+// The in-plane and temporal neighbours ("sources") of a voxel column: s = 0..7
+// the 3 x 3 neighbourhood in row-major order without its centre, 8 and 9 the
+// same column in frames f - 1 and f + 1.
+__device__ __forceinline__ void source_step(int s, int &dy, int &dx)
+{
+    const int o = s < 4 ? s : s + 1;
+    dy = o / 3 - 1;
+    dx = o - 3 * (dy + 1) - 1;
+}
+
+// sources of column (j, k) of frame f that lie inside the object, as bits
+__device__ __forceinline__ int sources_inside(int j, int k, int f, int NX, int NY, int NT)
+{
+    int m = 0x3FF;
+    if (j == 0) m &= ~0x007;
+    if (j == NY - 1) m &= ~0x0E0;
+    if (k == 0) m &= ~0x029;
+    if (k == NX - 1) m &= ~0x094;
+    if (f == 0) m &= ~0x100;
+    if (f == NT - 1) m &= ~0x200;
+    return m;
+}
+
+// r = h mod d for 1 <= d <= 2^16, in 32-bit steps
+__device__ __forceinline__ unsigned mod_small(uint64_t h, unsigned d)
+{
+    const unsigned hi = (unsigned)(h >> 32), lo = (unsigned)h;
+    return ((hi % d) * ((0xFFFFFFFFu % d + 1u) % d) + lo % d) % d;
 }
 
 // Update the voxel columns of super-voxel (sx, sy) of frame f; the whole CTA
-// cooperates (see the file comment for the four passes per column).
-// KW: 16-byte words per A record (1, 2, 3 for voxel scale 1, 2, 4);
-// kUnroll: views whose records and sinogram entries are in flight together;
+// cooperates (see the file comment for the passes of a column).
 // VEC: consecutive detector rows one lane owns (4 when N_t % 4 == 0, else 2);
-// kStaged: the column's records are read from shared memory (srec: two
-// buffers of stage_words words), the next column's copied in by a TMA bulk copy
-// while the current one is updated, so the theta pass waits on one global
-// round trip per view group instead of two and the apply pass on none.
+// kStaged: a column's records arrive in shared memory by a TMA bulk copy (srec:
+// two buffers) and are unpacked into entry lists while the column before it is
+// solved; else the lists are unpacked from global memory, in blocks of views;
+// kTile: the neighbours' values are read from the tile in shared memory
+// (stage_tile), else from x;
 // kHuber: 0 the quadratic data term, 1 the generalised Huber one
-// (XT_VoxUpdate.c:68-82), 2 decided per problem at run time (K.huber).
-template <int KW, int kUnroll, int VEC, bool kStaged, int kHuber>
+// (XT_VoxUpdate.c:68-82), 2 decided per problem at run time (K.huber);
+// kBatch: entries of a lane in flight together.
+//
+// A view's entries are read (theta) and reduced into (apply) by the same lane
+// for every column of the SV, so no barrier is needed between one column's
+// apply pass and the next one's theta loads.
+template <int VEC, bool kStaged, bool kTile, int kHuber, int kBatch>
 __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L, const IcdConst &K,
                                               const uint32_t *__restrict__ table,
                                               const int32_t *__restrict__ view_first,
                                               const uint8_t *__restrict__ mask, float *__restrict__ x,
                                               float *__restrict__ err, const float *__restrict__ wgt,
                                               float *__restrict__ mag, int f, int sx, int sy, IcdSmem &S,
-                                              IcdCount &cnt, uint32_t *srec, int stage_words)
+                                              IcdCount &cnt, uint32_t *dyn)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, W = blockDim.x >> 5;
     const int NX = g.N_x, NY = g.N_y, NZ = g.N_z, NT = g.N_t, MZ = g.z_overlap;
     const int nxy = NX * NY;
     const int RW = g.rec_words;
+    uint32_t *srec = dyn;
+    uint2 *lists = reinterpret_cast<uint2 *>(dyn + (kStaged ? 2 * L.stage_words : 0));
+    float *tile = reinterpret_cast<float *>(dyn + (kStaged ? 2 * L.stage_words : 0) + L.list_words) + 4;
     // A voxel column is updated in chunks of at most 32 detector rows (32 / MZ
     // voxel slices, one per lane of warp 0); chunk k covers rows [32k, 32k + 32)
     // and slices [k CZ, k CZ + CZ). Columns of up to 32 rows are one chunk.
@@ -369,34 +453,47 @@ __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L,
     const int n_chunks = (NT + 31) / 32;
 
     // lane -> (view group, run of VEC detector rows) for the theta / apply passes
-    using VT = typename VecF<VEC>::T;
-    const int lpr = CT / VEC;  // lanes per sinogram row of a full chunk
-    int lprp = 1;
-    while (lprp < lpr) lprp <<= 1;
+    const int lprp = icd_lanes_per_row(NT, VEC);
     const int G = 32 / lprp;  // view groups per warp
     const int grp = lane / lprp, tq = lane % lprp;
     const int t0 = tq * VEC;  // first detector row of this lane within the chunk
     const int gstride = W * G;
-    const int gfirst = warp * G + grp;
+    // lane -> (neighbour source, slice) for the neighbourhood pass: a short
+    // column leaves room for several sources side by side in a warp. The last
+    // warps take the first in-plane sources (warp 0 has the solve to do), warps
+    // from the second on the temporal ones.
+    int zp = 1;
+    while (zp < CZ) zp <<= 1;
+    const int nsub = 32 / zp, sub = lane / zp, zlane = lane % zp;
+    const int sfirst = (W - 1 - warp) * nsub, sstride = W * nsub;
+    const int ts = (warp - (W >= 4 ? 1 : 0)) * nsub + sub;  // temporal source 8 + ts
+    const int sv = L.sv, TW = sv + 2;  // the tile: the SV's columns and their in-plane neighbours
     const int fv0 = view_first[f], nv = view_first[f + 1] - fv0;
     const int iter = L.iter_dev ? *L.iter_dev : L.iter;  // 1-based iteration number
+    const bool no_skip = !L.zero_skipping || iter <= 1;
+    // entry lists: one per view group; two sets when staged (the current
+    // column's and the next one's). Unstaged, the lists hold blocks of
+    // L.block_views views.
+    const int cap = L.list_cap, set_slots = gstride * cap;
+    const uint32_t *rec_frame = table + (size_t)fv0 * nxy * RW;
 
     // ---- the SV's columns inside the reconstruction circle, shuffled ----------
     if (warp == 0) {
-        const int ncand = L.sv * L.sv;
+        const int ncand = sv * sv;
         int n = 0;
         for (int base = 0; base < ncand; base += 32) {
             const int i = base + lane;
-            int ok = 0, c = 0;
+            int ok = 0, c = 0, cell = 0;
             if (i < ncand) {
-                const int j = sy * L.sv + i / L.sv, k = sx * L.sv + i % L.sv;
+                const int j = sy * sv + i / sv, k = sx * sv + i % sv;
                 if (j < NY && k < NX) {
                     c = j * NX + k;
+                    cell = ((i / sv + 1) * TW + i % sv + 1) << 10 | sources_inside(j, k, f, NX, NY, g.N_time);
                     ok = mask[c] && (!L.sel || L.sel[(size_t)f * nxy + c]);
                 }
             }
             const unsigned m = __ballot_sync(0xffffffffu, ok);
-            if (ok) S.order[n + __popc(m & ((1u << lane) - 1))] = c;
+            if (ok) S.order[n + __popc(m & ((1u << lane) - 1))] = make_int2(c, cell);
             n += __popc(m);
         }
         __syncwarp();
@@ -405,8 +502,8 @@ __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L,
                                              (uint64_t)(sy * L.n_sv_x + sx)));
             for (int i = n - 1; i > 0; i--) {  // Fisher-Yates
                 h = mix64(h);
-                const int r = (int)(h % (uint64_t)(i + 1));
-                const int t = S.order[i];
+                const int r = (int)mod_small(h, (unsigned)(i + 1));
+                const int2 t = S.order[i];
                 S.order[i] = S.order[r];
                 S.order[r] = t;
             }
@@ -415,269 +512,409 @@ __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L,
     }
     __syncthreads();
     const int ncols = S.ncols;
-    const size_t rec_frame = (size_t)fv0 * nxy;
-    if (kStaged && ncols > 0)
-        stage_records(srec, table + (rec_frame + (size_t)S.order[0] * nv) * RW, nv * RW, &S.stage_bar[0]);
+    if (ncols == 0) return;
+    const bool starter = (int)threadIdx.x == 32 * (W - 1);  // starts the copies (not in warp 0, which solves)
+    const bool tile_copy = kTile && NZ % 4 == 0;
+    if (tile_copy) {
+        // the tile's rows are contiguous in x: one bulk copy each, on the first
+        // record buffer's mbarrier
+        if (warp == W - 1) stage_tile(tile, x, g, f, sx, sy, sv, nv * RW * 4, &S.stage_bar[0]);
+    } else if (kTile) {
+        const int cells = 3 * TW * TW;
+        for (int i = threadIdx.x; i < cells * NZ; i += blockDim.x) {
+            const int cell = i / NZ, z = i - cell * NZ;
+            const int p = cell / (TW * TW), r = cell - p * TW * TW;
+            const int ff = p == 0 ? f : p == 1 ? f - 1 : f + 1, j = sy * sv - 1 + r / TW, k = sx * sv - 1 + r % TW;
+            if (ff >= 0 && ff < g.N_time && j >= 0 && j < NY && k >= 0 && k < NX &&
+                (p == 0 || (r / TW >= 1 && r / TW <= sv && r % TW >= 1 && r % TW <= sv)))
+                tile[i] = x[((size_t)ff * nxy + (size_t)(j * NX + k)) * NZ + z];
+        }
+    }
+    // copy column ci's records into buffer ci mod 2
+    auto stage = [&](int ci) {
+        if (starter && ci < ncols) {
+            unsigned long long *bar = &S.stage_bar[ci & 1];
+            if (ci > 0 || !tile_copy) expect_bytes(bar, nv * RW * 4);
+            S.issued[ci & 1]++;
+            if (nv) bulk_copy(srec + (ci & 1) * L.stage_words, rec_frame + (size_t)S.order[ci].x * nv * RW, 4u * (unsigned)(nv * RW), bar);
+        }
+    };
+    if (kStaged) stage(0);
 
-    for (int ci = 0; ci < ncols; ci++) {
-        const int c = S.order[ci];
-        const int j = c / NX, k = c - j * NX;
+    // filter coefficients (with the 1 / sigma^q) of the neighbours at distance 1,
+    // sqrt 2 and sqrt 3
+    const float f1 = K.sf[9 + 1] * K.issq, f2 = K.sf[9] * K.issq, f3 = K.sf[0] * K.issq;
+
+    int2 next = make_int2(0, 0);
+    // ci = -1 only unpacks the first column's records
+    for (int ci = kStaged ? -1 : 0; ci < ncols; ci++) {
+        const int2 col = kStaged ? next : S.order[ci];
+        if (kStaged && ci + 1 < ncols) next = S.order[ci + 1];
+        const int c = col.x, inside = col.y & 0x3FF;
         const size_t col_off = ((size_t)f * nxy + c) * NZ;
-        const uint32_t *col_rec = kStaged ? srec + (ci & 1) * stage_words : table + (rec_frame + (size_t)c * nv) * RW;
+        float *cb = kTile ? tile + (col.y >> 10) * NZ : x + col_off;  // the column's values
+        const uint2 *ent = lists + (kStaged ? (ci & 1) * set_slots : 0) + (warp * G + grp) * cap;
 
         for (int ch = 0; ch < n_chunks; ch++) {
             const int z0 = ch * CZ;                                  // first slice of the chunk
             const int cz = NZ - z0 < CZ ? NZ - z0 : CZ;              // slices in the chunk
-            const int ct = cz * MZ;                                  // detector rows in the chunk
             const int rbase = ch * 32;                               // first detector row of the chunk
-            const bool zl = lane < cz;
-            const int z = z0 + lane;                                 // this lane's slice
-            const bool row_ok = tq < ct / VEC;
-
-            // ---- 1. neighbourhood (sources split over warps) + column activity ------
-            int active_pred;
-            const float V = zl ? x[col_off + z] : 0.0f;  // the column itself (warp 0 reuses it in the solve)
-            {
-                float num = 0.0f, den = 0.0f;
-                int pos = 0;
-                for (int s = warp; s < 10; s += W) {
-                    if (s < 8) {
-                        const int o = s < 4 ? s : s + 1;  // skip the centre of the 3x3
-                        const int dy = o / 3 - 1, dx = o % 3 - 1;
-                        const int jj = j + dy, kk = k + dx;
-                        const bool valid = jj >= 0 && jj < NY && kk >= 0 && kk < NX;
-                        const size_t noff = ((size_t)f * nxy + jj * NX + kk) * NZ;
-                        const float nz0 = (valid && zl) ? x[noff + z] : 0.0f;
-                        float nzm = __shfl_up_sync(0xffffffffu, nz0, 1);
-                        float nzp = __shfl_down_sync(0xffffffffu, nz0, 1);
-                        // across chunk edges the z +- 1 neighbours are outside the warp
-                        if (lane == 0 && z > 0 && valid) nzm = x[noff + z - 1];
-                        if (lane == cz - 1 && z + 1 < NZ && valid) nzp = x[noff + z + 1];
-                        if (valid && zl) {
-                            const float nb[3] = {nzm, nz0, nzp};
+            const bool row_ok = tq < cz * MZ / VEC;
+            const unsigned rows0 = (unsigned)(rbase + t0);           // this lane's rows within an entry
+            bool active = ci >= 0;
+            float V = 0.0f;
+            int vb = 0;
+            // (unstaged: the lists hold a block of the column's views at a time)
+            auto next_block = [&]() {
+                __syncwarp();
+                unpack_records<kBatch>(rec_frame + (size_t)c * nv * RW, RW, NT, K.dt, lists + (warp * G + grp) * cap,
+                                       warp * G + grp, gstride, vb, min(vb + L.block_views, nv), tq, lprp);
+                __syncwarp();
+            };
+            if (ci >= 0) {
+                const bool zl = zlane < cz;
+                const int z = z0 + zlane;  // this lane's slice
+                const float v0 = kTile || zl ? cb[z] : 0.0f;
+                V = zl ? v0 : 0.0f;
+                const bool sure = no_skip || __any_sync(0xffffffffu, zl && V != 0.0f);
+                // theta's first batch of entries is in flight during the
+                // neighbourhood pass (e and w keep the last values loaded: an entry
+                // that is not there has weight zero)
+                Rows<VEC> e[kBatch], w[kBatch];
+                float na[kBatch];
+                f32x2 t1[VEC / 2], t2[VEC / 2];
 #pragma unroll
-                            for (int dz = -1; dz <= 1; dz++) {
-                                const int zz = z + dz;
-                                if (zz < 0 || zz >= NZ) continue;
-                                const float n = nb[dz + 1];
-                                const float b = qg_weight(V - n, K.q, K.qmp, K.issq, K.issqp, K.cs, K.bs0);
-                                const float cf = K.sf[(dz + 1) * 9 + (dy + 1) * 3 + (dx + 1)] * b;
-                                num += cf * n;
-                                den += cf;
-                                pos |= n > 0.0f;
+                for (int u = 0; u < kBatch; u++) e[u] = w[u] = Rows<VEC>{};
+#pragma unroll
+                for (int i = 0; i < VEC / 2; i++) t1[i] = t2[i] = 0ull;
+                if (!kStaged) next_block();
+                int n_ent = row_ok ? (int)ent[0].x : 0, n_warp = (int)ent[0].y, i0 = 0;
+                bool first = true;
+                for (;;) {
+                    // entries i0 .. i0 + kBatch - 1: all loads in flight together
+#pragma unroll
+                    for (int u = 0; u < kBatch; u++) {
+                        const uint2 en = ent[1 + i0 + u];
+                        const unsigned off = en.x + rows0;
+                        na[u] = __uint_as_float(en.y);
+                        load_entry(e[u], w[u], err + off, wgt + off, i0 + u, n_ent);
+                    }
+                    // ---- 1. neighbourhood, while the first batch arrives (sources
+                    //         split over warps and lane groups) ------------------------
+                    if (first) {
+                        first = false;
+                        float num = 0.0f, den = 0.0f, top = 0.0f;  // top: the largest neighbour, or 0
+                        const bool zm = z > 0, zn = z + 1 < NZ;
+                        for (int s0 = sfirst; s0 < 8; s0 += sstride) {  // in-plane; uniform over the warp
+                            const int s = min(s0 + sub, 7);
+                            int dy, dx;
+                            source_step(s, dy, dx);
+                            const bool ok = zl && s0 + sub < 8 && ((inside >> s) & 1), side = dy == 0 || dx == 0;
+                            const float *src = cb + (ptrdiff_t)((dy * (kTile ? TW : NX) + dx) * NZ);
+                            float n[3], d[3], fl[3], cf[3];
+                            // (in the tile every address read exists: values outside the
+                            // object are dropped after the load, without a branch)
+                            const float nm = kTile || (ok && zm) ? src[z - 1] : 0.0f;
+                            const float n0 = kTile || ok ? src[z] : 0.0f;
+                            const float np = kTile || (ok && zn) ? src[z + 1] : 0.0f;
+                            n[0] = ok && zm ? nm : 0.0f;
+                            n[1] = ok ? n0 : 0.0f;
+                            n[2] = ok && zn ? np : 0.0f;
+                            const float fo = side ? f2 : f3;
+                            fl[0] = ok && zm ? fo : 0.0f;
+                            fl[1] = ok ? (side ? f1 : f2) : 0.0f;
+                            fl[2] = ok && zn ? fo : 0.0f;
+#pragma unroll
+                            for (int i = 0; i < 3; i++) d[i] = V - n[i];
+                            qg_coef(d, fl, K.q, K.qmp, K.issqp, K.cs, K.qocs, cf);
+#pragma unroll
+                            for (int i = 0; i < 3; i++) {
+                                num += cf[i] * n[i];
+                                den += cf[i];
+                                top = fmaxf(top, n[i]);
                             }
                         }
-                    } else {
-                        const int ff = f + (s == 8 ? -1 : 1);
-                        if (ff >= 0 && ff < g.N_time && zl) {
-                            const float n = x[((size_t)ff * nxy + c) * NZ + z];
-                            const float b = qg_weight(V - n, K.q, K.qmp, K.istq, K.istqp, K.ct, K.bt0);
-                            const float cf = K.tf * b;
-                            num += cf * n;
-                            den += cf;
-                            pos |= n > 0.0f;
+                        // temporal (the same source for every lane of a lane group)
+                        for (int t0_ = ts - sub; t0_ < 2 && t0_ >= 0; t0_ += sstride) {
+                            const int t = min(t0_ + sub, 1);
+                            const bool ok = zl && t0_ + sub < 2 && ((inside >> (8 + t)) & 1);
+                            const float *src = kTile ? cb + (t + 1) * TW * TW * NZ
+                                                     : cb + (t == 0 ? -(ptrdiff_t)nxy : (ptrdiff_t)nxy) * NZ;
+                            const float n0 = kTile || ok ? src[z] : 0.0f;
+                            const float n[1] = {ok ? n0 : 0.0f}, d[1] = {V - n[0]}, fl[1] = {ok ? K.tf * K.istq : 0.0f};
+                            float cf[1];
+                            qg_coef(d, fl, K.q, K.qmp, K.istqp, K.ct, K.qoct, cf);
+                            num += cf[0] * n[0];
+                            den += cf[0];
+                            top = fmaxf(top, n[0]);
+                        }
+                        unsigned pw = __ballot_sync(0xffffffffu, top > 0.0f);
+                        for (int off = zp; off < 32; off <<= 1) {
+                            num += __shfl_xor_sync(0xffffffffu, num, off);
+                            den += __shfl_xor_sync(0xffffffffu, den, off);
+                            pw |= pw >> off;
+                        }
+                        if (sub == 0) S.nd[warp][zlane] = make_float2(num, den);
+                        if (lane == 0) S.pos[warp] = pw & (0xffffffffu >> (32 - zp));
+                        // a column that may be inactive (all of it zero) needs the
+                        // neighbours' verdict first (uniform: every warp read the column)
+                        if (!sure) {
+                            __syncthreads();
+                            unsigned any = 0;
+                            for (int q = 0; q < W; q++) any |= S.pos[q];
+                            active = any != 0;
+                            if (!active) break;
                         }
                     }
-                }
-                S.num[warp][lane] = num;
-                S.den[warp][lane] = den;
-                S.pos[warp][lane] = pos;
-                // a column is skipped only if every slice is zero with no positive
-                // neighbour (in-column neighbours are the column's own values)
-                active_pred = !L.zero_skipping || iter <= 1 || (zl && V != 0.0f) || pos;
-            }
-            // ---- 2. theta over the column's views. When the column is surely
-            //         active (zero skipping off or in its first iteration, or a
-            //         nonzero slice: the same test in every warp, as every warp
-            //         read the column), theta runs before the barrier that also
-            //         publishes the neighbourhood sums, so its loads go out without
-            //         waiting for the other warps; otherwise after it, and only
-            //         for an active column -------------------------------------------
-            bool recs_ok = true;
-            if (kStaged && ch == 0)  // issued one column earlier
-                recs_ok = wait_staged(&S.stage_bar[ci & 1], cnt.phases, ci & 1, cnt.timeouts, S.abort, S.abort_bar,
-                                      S.abort_parity);
-            const bool sure = !L.zero_skipping || iter <= 1 || __any_sync(0xffffffffu, zl && V != 0.0f);
-            // a thread whose wait gave up reads no record (their headers address
-            // the sinogram); the CTA leaves after the barrier
-            if (sure)
-                theta_column<KW, kUnroll, VEC, kStaged, kHuber>(K, col_rec, err, wgt, gfirst, gstride, nv, RW, NT,
-                                                               rbase + t0, row_ok && recs_ok, lprp, grp, t0, warp, S);
-            const int any_active = __syncthreads_or(active_pred);
-            if (ch == 0) {
-                // a late copy leaves this column's records undefined: no update, no
-                // further copies (S.abort is read after the barrier, so uniformly)
-                if (kStaged && S.abort) return;
-                // every thread is past the previous column's apply pass: its record
-                // buffer may be refilled with the next column's
-                if (kStaged && ci + 1 < ncols)
-                    stage_records(srec + ((ci + 1) & 1) * stage_words,
-                                  table + (rec_frame + (size_t)S.order[ci + 1] * nv) * RW, nv * RW,
-                                  &S.stage_bar[(ci + 1) & 1]);
-            }
-            if (!any_active) {
-                if (warp == 0 && zl) cnt.skip++;
-                if (warp == 0 && lane == 0 && ch == 0) mag[(size_t)f * nxy + c] = 0.0f;
-                continue;  // uniform across the CTA
-            }
-            if (!sure) {  // uniform across the CTA
-                theta_column<KW, kUnroll, VEC, kStaged, kHuber>(K, col_rec, err, wgt, gfirst, gstride, nv, RW, NT,
-                                                               rbase + t0, row_ok && recs_ok, lprp, grp, t0, warp, S);
-                __syncthreads();
-            }
-
-            // ---- 3. zero-skipping and solve (warp 0, lane = slice of the chunk) ------
-            if (warp == 0) {
-                const float V0 = V;
-                float numA = 0.0f, denA = 0.0f, t1 = 0.0f, t2 = 0.0f;
-                int pos = 0;
-                for (int w = 0; w < W; w++) {
-                    numA += S.num[w][lane];
-                    denA += S.den[w][lane];
-                    pos |= S.pos[w][lane];
-                    if (lane < ct) {
-                        t1 += S.th1[w][lane];
-                        t2 += S.th2[w][lane];
-                    }
-                }
-                // in-column z - 1 / z + 1: the chunk below is already updated
-                // (Gauss-Seidel over the chunks), the chunk above not yet
-                const float edge_m = (z0 > 0) ? x[col_off + z0 - 1] : 0.0f;
-                const float edge_p = (z0 + cz < NZ) ? x[col_off + z0 + cz] : 0.0f;
-                {
-                    float vm = __shfl_up_sync(0xffffffffu, V0, 1);
-                    float vp = __shfl_down_sync(0xffffffffu, V0, 1);
-                    if (lane == 0) vm = edge_m;
-                    if (lane == cz - 1) vp = edge_p;
-                    if (z >= 1 && vm > 0.0f) pos = 1;
-                    if (z + 1 < NZ && vp > 0.0f) pos = 1;
-                }
-                const bool skip = !zl || (L.zero_skipping && iter > 1 && V0 == 0.0f && !pos);
-                __syncwarp();
-                S.th1[0][lane] = t1;
-                S.th2[0][lane] = t2;
-                __syncwarp();
-                float th1 = 0.0f, th2 = 0.0f;
-                if (zl)
-                    for (int r = 0; r < MZ; r++) {
-                        th1 += S.th1[0][lane * MZ + r];
-                        th2 += S.th2[0][lane * MZ + r];
-                    }
-                float cur = V0;
+                    // ---- 2. theta1 = -sum a w e, theta2 = sum a^2 w over the column's
+                    //         entries (XT_VoxUpdate.c:56-85) ---------------------------
 #pragma unroll
-                for (int parity = 0; parity < 2; parity++) {
-                    float vm = __shfl_up_sync(0xffffffffu, cur, 1);
-                    float vp = __shfl_down_sync(0xffffffffu, cur, 1);
-                    if (lane == 0) vm = edge_m;
-                    if (lane == cz - 1) vp = edge_p;
-                    if (!skip && (z & 1) == parity) {
-                        float num = numA, den = denA;
-                        if (z >= 1) {
-                            const float cf = K.sf[0 * 9 + 4] * qg_weight(V0 - vm, K.q, K.qmp, K.issq, K.issqp, K.cs, K.bs0);
-                            num += cf * vm;
-                            den += cf;
+                    for (int u = 0; u < kBatch; u++) {
+                        const f32x2 a = pack2(na[u], na[u]);
+#pragma unroll
+                        for (int i = 0; i < VEC / 2; i++) {
+                            f32x2 ww = w[u].p[i];
+                            if (kHuber == 1 || (kHuber == 2 && K.huber)) {
+                                float w0, w1, e0, e1;
+                                unpack2(ww, w0, w1);
+                                unpack2(e[u].p[i], e0, e1);
+                                // |e sqrt(w)| >= T only if e^2 w >= T^2 up to rounding: most
+                                // entries need no square root
+                                if (!(e0 * e0 * w0 < K.huber_T2 && w0 >= 0.0f && e1 * e1 * w1 < K.huber_T2 && w1 >= 0.0f)) {
+                                    const float s0 = sqrtf(w0), s1 = sqrtf(w1);
+                                    if (!(fabsf(e0 * s0) < K.huber_T)) w0 = K.huber_T * K.huber_delta * s0 / fabsf(e0);
+                                    if (!(fabsf(e1 * s1) < K.huber_T)) w1 = K.huber_T * K.huber_delta * s1 / fabsf(e1);
+                                    ww = pack2(w0, w1);
+                                }
+                            }
+                            const f32x2 aw = mul2(a, ww);  // -a w
+                            t2[i] = fma2(a, aw, t2[i]);
+                            t1[i] = fma2(e[u].p[i], aw, t1[i]);
                         }
-                        if (z + 1 < NZ) {
-                            const float cf = K.sf[2 * 9 + 4] * qg_weight(V0 - vp, K.q, K.qmp, K.issq, K.issqp, K.cs, K.bs0);
-                            num += cf * vp;
-                            den += cf;
-                        }
-                        const float u = (num + th2 * V0 - th1) / (den + th2);
-                        cur = V0 + K.alpha * (u - V0);
+                    }
+                    i0 += kBatch;
+                    if (i0 >= n_warp) {  // uniform over the warp
+                        vb += L.block_views;
+                        if (kStaged || vb >= nv) break;
+                        next_block();
+                        n_ent = row_ok ? (int)ent[0].x : 0;
+                        n_warp = (int)ent[0].y;
+                        i0 = 0;
                     }
                 }
-                const float dx = skip ? 0.0f : cur - V0;
-                S.dx[lane] = dx;
-                if (zl) {
-                    if (!skip) {
-                        x[col_off + z] = cur;
-                        cnt.upd++;
-                        cnt.sum_dx += fabsf(dx);
-                        cnt.sum_x += fabsf(cur);
-                    } else {
-                        cnt.skip++;
+                if (active) {
+                    // sum over the warp's view groups: two groups share out their rows
+                    // until a lane holds one row, then add it up over the rest
+                    float a[VEC], b[VEC];
+#pragma unroll
+                    for (int i = 0; i < VEC / 2; i++) {
+                        unpack2(t1[i], a[2 * i], a[2 * i + 1]);
+                        unpack2(t2[i], b[2 * i], b[2 * i + 1]);
                     }
-                }
-                float m = fabsf(dx);
-                for (int off = 16; off > 0; off >>= 1) m += __shfl_xor_sync(0xffffffffu, m, off);
-                if (lane == 0) {
-                    float *mp = mag + (size_t)f * nxy + c;
-                    *mp = ch == 0 ? m : *mp + m;
+                    int row = t0, off = lprp;
+#pragma unroll
+                    for (int n = VEC / 2; n >= 1; n /= 2) {
+                        const bool up = (lane & off) != 0;
+#pragma unroll
+                        for (int i = 0; i < n; i++) {
+                            const float sa = up ? a[i] : a[n + i], sb = up ? b[i] : b[n + i];
+                            a[i] = (up ? a[n + i] : a[i]) + __shfl_xor_sync(0xffffffffu, sa, off);
+                            b[i] = (up ? b[n + i] : b[i]) + __shfl_xor_sync(0xffffffffu, sb, off);
+                        }
+                        row += up ? n : 0;
+                        off <<= 1;
+                    }
+                    const bool writes = lane < off && row_ok;
+                    for (; off < 32; off <<= 1) {
+                        a[0] += __shfl_xor_sync(0xffffffffu, a[0], off);
+                        b[0] += __shfl_xor_sync(0xffffffffu, b[0], off);
+                    }
+                    if (writes) S.th[warp][row] = make_float2(a[0], b[0]);
                 }
             }
             __syncthreads();
 
-            // ---- 4. apply e -= a dx (the next chunk's or column's barrier orders
-            //         these reductions before its theta loads) ---------------------------
+            // while warp 0 solves, the other warps unpack the next column's records
+            // (warp 1 also warp 0's share), and the copy of the column after it
+            // starts, into the buffer that the current column's were unpacked from
+            if (kStaged && (ch == n_chunks - 1 || ci < 0) && ci + 1 < ncols) {
+                const int b = (ci + 1) & 1;
+                stage(ci + 2);
+                if ((warp > 0 || W == 1 || ci < 0) &&
+                    wait_staged(&S.stage_bar[b], cnt.phases, b, cnt.timeouts, S.abort) && (warp > 0 || W == 1)) {
+                    for (int q = warp; q >= 0; q = q == 1 ? 0 : -1)
+                        unpack_records<kBatch>(srec + b * L.stage_words, RW, NT, K.dt,
+                                               lists + b * set_slots + (q * G + grp) * cap, q * G + grp, gstride, 0, nv, tq,
+                                               lprp);
+                }
+                cnt.phases ^= 1u << b;
+            }
+
+            // ---- 3. zero-skipping and solve (warp 0, lane = slice of the chunk) --------
+            if (warp == 0 && ci >= 0) {
+                const bool sl = lane < cz;
+                if (!active) {
+                    if (sl) cnt.skip++;
+                    if (lane == 0 && ch == 0) mag[(size_t)f * nxy + c] = 0.0f;
+                } else {
+                    const int sz = z0 + lane;
+                    const bool has_m = sl && sz >= 1, has_p = sl && sz + 1 < NZ;
+                    const float fv[2] = {has_m ? f1 : 0.0f, has_p ? f1 : 0.0f};
+                    // in-column z - 1 / z + 1: the chunk below is already updated
+                    // (Gauss-Seidel over the chunks), the chunk above not yet
+                    float vm = has_m ? cb[sz - 1] : 0.0f, vp = has_p ? cb[sz + 1] : 0.0f;
+                    float numA = 0.0f, denA = 0.0f, th1 = 0.0f, th2 = 0.0f;
+                    unsigned pw = 0;
+#pragma unroll 4
+                    for (int q = 0; q < W; q++) {
+                        const float2 nd = S.nd[q][lane], th = S.th[q][lane];
+                        numA += nd.x;
+                        denA += nd.y;
+                        th1 += th.x;
+                        th2 += th.y;
+                        pw |= S.pos[q];
+                    }
+                    const bool pos = ((pw >> lane) & 1u) || vm > 0.0f || vp > 0.0f;
+                    const bool skip = !sl || (!no_skip && V == 0.0f && !pos);
+                    if (MZ > 1) {  // a slice covers MZ detector rows
+                        __syncwarp();
+                        S.th[0][lane] = make_float2(th1, th2);
+                        __syncwarp();
+                        th1 = th2 = 0.0f;
+                        if (sl)
+                            for (int r = 0; r < MZ; r++) {
+                                const float2 th = S.th[0][lane * MZ + r];
+                                th1 += th.x;
+                                th2 += th.y;
+                            }
+                    }
+                    // even slices, then odd ones against the even ones' new values (the
+                    // other lanes' results are dropped)
+                    float cur = V;
+#pragma unroll 1
+                    for (int parity = 0; parity < 2; parity++) {
+                        const float d[2] = {V - vm, V - vp};
+                        float cv[2];
+                        qg_coef(d, fv, K.q, K.qmp, K.issqp, K.cs, K.qocs, cv);
+                        if (!skip && (sz & 1) == parity) {
+                            const float num = (numA + cv[0] * vm) + cv[1] * vp;
+                            const float den = (denA + cv[0]) + cv[1];
+                            const float u = (num + th2 * V - th1) / (den + th2);
+                            cur = V + K.alpha * (u - V);
+                        }
+                        const float um = __shfl_up_sync(0xffffffffu, cur, 1), up = __shfl_down_sync(0xffffffffu, cur, 1);
+                        if (has_m && lane > 0) vm = um;  // across chunk edges: the values read above
+                        if (has_p && lane < cz - 1) vp = up;
+                    }
+                    const float dx = skip ? 0.0f : cur - V;
+                    S.dx[lane] = MZ == 1 ? dx : __shfl_sync(0xffffffffu, dx, lane / MZ);
+                    if (sl && !skip) {
+                        x[col_off + sz] = cur;
+                        if (kTile) cb[sz] = cur;
+                        cnt.upd++;
+                        cnt.sum_dx += fabsf(dx);
+                        cnt.sum_x += fabsf(cur);
+                    }
+                    if (sl && skip) cnt.skip++;
+                }
+            }
+            __syncthreads();
+            // a late copy leaves the next column's records undefined: no further
+            // update, no further copies (uniform: the flag was set before the barrier)
+            if (S.abort) return;
+            if (ci < 0) break;
+            if (!active) continue;
+
+            // ---- 4. apply e -= a dx ------------------------------------------------------
             {
-                float dxv[VEC];
+                Rows<VEC> dxv{};
+                if (row_ok) dxv = *reinterpret_cast<const Rows<VEC> *>(&S.dx[t0]);
                 bool any = false;
 #pragma unroll
-                for (int i = 0; i < VEC; i++) {
-                    dxv[i] = row_ok ? S.dx[(t0 + i) / MZ] : 0.0f;
-                    any |= dxv[i] != 0.0f;
-                }
+                for (int i = 0; i < VEC / 2; i++) any |= (dxv.p[i] & 0x7FFFFFFF7FFFFFFFull) != 0;
+                any = __any_sync(0xffffffffu, any);
                 if (any) {
-                    for (int v0 = gfirst; v0 < nv; v0 += kUnroll * gstride) {
-                        Rec<KW> R[kUnroll];
+                    for (vb = 0;;) {
+                        if (!kStaged && L.block_views < nv) next_block();
+                        const int n = row_ok ? (int)ent[0].x : 0, n_warp = (int)ent[0].y;
+                        for (int i0 = 0; i0 < n_warp; i0 += 4) {  // uniform over the warp
 #pragma unroll
-                        for (int u = 0; u < kUnroll; u++) {
-                            const int v = v0 + u * gstride;
-                            if (v < nv) R[u] = kStaged ? load_rec_smem<KW>(col_rec + (size_t)v * RW)
-                                                   : load_rec<KW>(col_rec + (size_t)v * RW);
-                            else R[u].w[0].x = 0u;
-                        }
+                            for (int u = 0; u < 4; u++) {
+                                const uint2 en = ent[1 + i0 + u];
+                                const float na = __uint_as_float(en.y);
+                                const f32x2 a = pack2(na, na);
+                                Rows<VEC> d;
 #pragma unroll
-                        for (int u = 0; u < kUnroll; u++) {
-                            const uint32_t hdr = R[u].w[0].x;
-                            const int cnt_q = hdr >> 24;
-                            const unsigned sb = (hdr & 0xFFFFFFu) * (unsigned)NT + (unsigned)(rbase + t0);
-#pragma unroll
-                            for (int q = 0; q < 4 * KW - 1; q++) {
-                                if (q < cnt_q) {
-                                    const float a = -(rec_val<KW>(R[u], q) * K.dt);
-                                    float d[VEC];
-#pragma unroll
-                                    for (int i = 0; i < VEC; i++) d[i] = a * dxv[i];
-                                    red_add(err + (sb + (unsigned)(q * NT)), d);
-                                }
+                                for (int q = 0; q < VEC / 2; q++) d.p[q] = mul2(a, dxv.p[q]);
+                                red_add(err + (en.x + rows0), d, i0 + u, n);
                             }
                         }
+                        vb += L.block_views;
+                        if (kStaged || vb >= nv) break;
+                    }
+                }
+                // the column's update magnitude: the sum over its slices of |dx| (by
+                // the last warp: warp 0's chain is the longest)
+                if (warp == W - 1) {
+                    float m = lane < cz * MZ && lane % MZ == 0 ? fabsf(S.dx[lane]) : 0.0f;
+                    for (int off = 16; off > 0; off >>= 1) m += __shfl_xor_sync(0xffffffffu, m, off);
+                    if (lane == 0) {
+                        float *mp = mag + (size_t)f * nxy + c;
+                        *mp = ch == 0 ? m : *mp + m;
                     }
                 }
             }
         }
     }
+    // the next SV's tile is written by the copy engine over these generic writes
+    if (kTile) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
 }  // namespace
 
+__device__ __forceinline__ void init_copies(IcdSmem &S)
+{
+    if (threadIdx.x == 0) {
+        S.abort = 0;
+        for (int b = 0; b < 2; b++) {
+            S.issued[b] = 0;
+            asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(&S.stage_bar[b]))
+                         : "memory");
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+}
+
+// After an abort, copies may still write into this CTA's shared memory: give
+// the last one of each buffer one more bounded wait before the CTA exits.
+__device__ __forceinline__ void drain_copies(IcdSmem &S)
+{
+    if (S.abort && threadIdx.x == 0)
+        for (int b = 0; b < 2; b++)
+            if (S.issued[b]) wait_parity_bounded(&S.stage_bar[b], (S.issued[b] - 1) & 1u);
+}
+
 // One colour phase of one problem: persistent CTAs drain the phase's SV queue.
-// With kStaged, the dynamic shared memory holds two record buffers of
-// stage_words words each (the current and the next column's A records).
-template <int KW, int kUnroll, int VEC, bool kStaged, int kHuber>
-__global__ void __launch_bounds__(kMaxWarps * 32, 4) icd_phase_kernel(
+// 128 registers a thread: four CTAs of four warps on an SM, which is what the
+// batch of loads in flight needs; at 72 registers (seven CTAs) the spills cost
+// more than the occupancy gave (4-D workload, iteration with its NH passes: 16.1
+// against 12.0 ms).
+template <int VEC, bool kStaged, bool kTile, int kHuber, int kBatch>
+__global__ void __launch_bounds__(kMaxWarps * 32, 2) icd_phase_kernel(
     Geom g, IcdLaunch L, IcdConst K, const uint32_t *__restrict__ table, const int32_t *__restrict__ view_first,
     const uint8_t *__restrict__ mask, float *__restrict__ x, float *__restrict__ err, const float *__restrict__ wgt,
-    float *__restrict__ mag, IcdStats *__restrict__ stats, unsigned int *__restrict__ queue, int stage_words)
+    float *__restrict__ mag, IcdStats *__restrict__ stats, unsigned int *__restrict__ queue)
 {
     __shared__ IcdSmem S;
-    extern __shared__ __align__(16) uint32_t s_rec[];
+    extern __shared__ __align__(16) uint32_t s_dyn[];
     const int KC = L.colors_k;
     const int hx = (L.n_sv_x + KC - 1) / KC, slots = hx * ((L.n_sv_y + KC - 1) / KC);
     const int n_items = L.items ? *L.n_items : g.N_time * slots;
     IcdCount cnt{};
-    if (threadIdx.x == 0) S.abort = 0;
-    if (kStaged && threadIdx.x == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(&S.stage_bar[0]))
-                     : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"((unsigned)__cvta_generic_to_shared(&S.stage_bar[1]))
-                     : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
+    init_copies(S);
     for (;;) {
         __syncthreads();  // S.item / S.order of the previous SV are no longer read
-        if (kStaged && S.abort) break;  // uniform: written before the barrier
+        if (S.abort) break;  // uniform: written before the barrier
         if (threadIdx.x == 0) S.item = (int)atomicAdd(queue, 1u);
         __syncthreads();
         const int item = S.item;
@@ -696,28 +933,58 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 4) icd_phase_kernel(
             sy = KC * (rem / hx) + color / KC;
         }
         if (sx >= L.n_sv_x || sy >= L.n_sv_y) continue;  // uniform
-        icd_update_sv<KW, kUnroll, VEC, kStaged, kHuber>(g, L, K, table, view_first, mask, x, err, wgt, mag, f, sx, sy,
-                                                         S,
-                                                 cnt, s_rec, stage_words);
+        icd_update_sv<VEC, kStaged, kTile, kHuber, kBatch>(g, L, K, table, view_first, mask, x, err, wgt, mag, f, sx, sy,
+                                                          S, cnt, s_dyn);
     }
-    // after an abort, the late copy may still write into this CTA's shared
-    // memory: give it one more bounded wait before the CTA exits
-    if (kStaged && S.abort && threadIdx.x == 0) wait_parity_bounded(&S.stage_bar[S.abort_bar], S.abort_parity);
+    drain_copies(S);
     flush_counts(cnt, stats);
 }
 
-// Record staging needs two buffers of (most views in a frame) x record words;
-// above this size the sweep reads records from global memory instead.
-constexpr int kMaxStageBytes = 16 * 1024;
+// Shared memory of a launch (the fields of L that describe it; returns whether
+// records are staged). Records and two sets of entry lists are staged up to
+// kMaxStageBytes; beyond (thousands of views in a frame) lists of kBlockBytes
+// are unpacked from global memory where they are used. An SV's neighbourhood tile
+// (three planes of (sv + 2)^2 columns) is kept up to kMaxTileBytes; beyond, the
+// neighbours are read from x where they are used.
+constexpr size_t kMaxStageBytes = 128 * 1024, kBlockBytes = 16 * 1024, kMaxTileBytes = 40 * 1024;
 
-template <int KW, int U, int VEC, bool kStaged, int kHuber>
-static void launch_staged(const Geom &g, const IcdLaunch &L, const IcdConst &K, const uint32_t *d_table,
-                          const int32_t *d_view_first, const uint8_t *d_mask, float *d_x, float *d_err,
-                          const float *d_w, float *d_mag, IcdStats *d_stats, unsigned int *d_queue, int stage_words,
-                          cudaStream_t st)
+// What a sweep keeps in shared memory: a block of entry lists only; or two record
+// buffers and the lists of two columns; or these and the SV's neighbourhood tile.
+enum IcdMode { ICD_PLAIN, ICD_STAGED, ICD_STAGED_TILE };
+static IcdMode icd_plan_shared(const Geom &g, IcdLaunch &L, int vec, int batch, IcdMode most = ICD_STAGED_TILE)
+{
+    const int gstride = L.warps * (32 / icd_lanes_per_row(g.N_t, vec));
+    const int vpg = std::max(1, (g.max_views + gstride - 1) / gstride);
+    L.stage_words = g.max_views * g.rec_words;
+    L.list_cap = icd_list_cap(vpg, g.kmax, batch);
+    L.block_views = vpg * gstride;
+    size_t lists = (size_t)gstride * L.list_cap * sizeof(uint2);
+    const size_t records = L.stage_words * sizeof(uint32_t);
+    const size_t tile = 3 * (size_t)(L.sv + 2) * (L.sv + 2) * g.N_z * sizeof(float);
+    IcdMode mode = ICD_PLAIN;
+    if (L.stage_records && most >= ICD_STAGED && 2 * (records + lists) <= kMaxStageBytes) {
+        mode = most == ICD_STAGED_TILE && tile <= kMaxTileBytes ? ICD_STAGED_TILE : ICD_STAGED;
+        lists *= 2;
+    } else if (lists > kBlockBytes) {
+        int v = vpg;
+        while (v > 1 && (size_t)gstride * icd_list_cap(v, g.kmax, batch) * sizeof(uint2) > kBlockBytes) v--;
+        L.list_cap = icd_list_cap(v, g.kmax, batch);
+        L.block_views = v * gstride;
+        lists = (size_t)gstride * L.list_cap * sizeof(uint2);
+    }
+    L.list_words = (int)((lists + 15) / 16 * 4);
+    L.shared_bytes = (mode != ICD_PLAIN ? 2 * (int)records : 0) + 4 * L.list_words + (mode == ICD_STAGED_TILE ? (int)tile + 64 : 0);
+    return mode;
+}
+
+template <int VEC, bool kStaged, bool kTile, int kHuber, int kBatch>
+static void launch_mode(const Geom &g, const IcdLaunch &L, const IcdConst &K, const uint32_t *d_table,
+                        const int32_t *d_view_first, const uint8_t *d_mask, float *d_x, float *d_err,
+                        const float *d_w, float *d_mag, IcdStats *d_stats, unsigned int *d_queue, cudaStream_t st)
 {
     const int threads = L.warps * 32;
-    const size_t smem = kStaged ? 2 * (size_t)stage_words * sizeof(uint32_t) : 0;
+    const size_t smem = (size_t)L.shared_bytes;
+    const auto kernel = icd_phase_kernel<VEC, kStaged, kTile, kHuber, kBatch>;
     // resident CTAs per SM, cached per (device, block size, shared memory) so a
     // launch being captured into a CUDA graph makes no occupancy query
     struct Occ {
@@ -740,8 +1007,8 @@ static void launch_staged(const Geom &g, const IcdLaunch &L, const IcdConst &K, 
             }
         if (!hit) {
             cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                &per_sm, icd_phase_kernel<KW, U, VEC, kStaged, kHuber>, threads, smem);
+            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kMaxStageBytes + kMaxTileBytes));
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
             cache.push_back({dev, threads, sms, per_sm, smem});
         }
     }
@@ -749,28 +1016,24 @@ static void launch_staged(const Geom &g, const IcdLaunch &L, const IcdConst &K, 
     long long grid = (long long)sms * (per_sm > 0 ? per_sm : 1);
     if (grid > items) grid = items;
     if (L.max_ctas > 0 && grid > L.max_ctas) grid = L.max_ctas;
-    icd_phase_kernel<KW, U, VEC, kStaged, kHuber><<<(unsigned)grid, threads, smem, st>>>(
-        g, L, K, d_table, d_view_first, d_mask, d_x, d_err, d_w, d_mag, d_stats, d_queue, stage_words);
+    kernel<<<(unsigned)grid, threads, smem, st>>>(g, L, K, d_table, d_view_first, d_mask, d_x, d_err, d_w, d_mag,
+                                                  d_stats, d_queue);
 }
 
-template <int KW, int U, int VEC>
-static void launch_kw(const Geom &g, const IcdLaunch &L, const IcdConst &K, const uint32_t *d_table,
-                      const int32_t *d_view_first, const uint8_t *d_mask, float *d_x, float *d_err, const float *d_w,
-                      float *d_mag, IcdStats *d_stats, unsigned int *d_queue, cudaStream_t st)
+template <int VEC, int kBatch>
+static void launch_vec(const Geom &g, const IcdLaunch &L_, const IcdConst &K, const uint32_t *d_table,
+                       const int32_t *d_view_first, const uint8_t *d_mask, float *d_x, float *d_err, const float *d_w,
+                       float *d_mag, IcdStats *d_stats, unsigned int *d_queue, cudaStream_t st)
 {
-    const int stage_words = g.max_views * g.rec_words;  // a multiple of 4 words: 16-byte aligned buffers
-    const bool staged = L.stage_records && 2 * (size_t)stage_words * sizeof(uint32_t) <= (size_t)kMaxStageBytes;
-#define MBIR_STAGED(S, H)                                                                                         \
-    launch_staged<KW, U, VEC, S, H>(g, L, K, d_table, d_view_first, d_mask, d_x, d_err, d_w, d_mag, d_stats, d_queue, \
-                                    S ? stage_words : 0, st)
-    if (staged) {
-        if (K.huber) MBIR_STAGED(true, 1);
-        else MBIR_STAGED(true, 0);
-    } else {
-        if (K.huber) MBIR_STAGED(false, 1);
-        else MBIR_STAGED(false, 0);
-    }
-#undef MBIR_STAGED
+    IcdLaunch L = L_;
+    const IcdMode mode = icd_plan_shared(g, L, VEC, kBatch);
+#define MBIR_MODE(S, T)                                                                                       \
+    (K.huber ? launch_mode<VEC, S, T, 1, kBatch> : launch_mode<VEC, S, T, 0, kBatch>)(                          \
+        g, L, K, d_table, d_view_first, d_mask, d_x, d_err, d_w, d_mag, d_stats, d_queue, st)
+    if (mode == ICD_STAGED_TILE) MBIR_MODE(true, true);
+    else if (mode == ICD_STAGED) MBIR_MODE(true, false);
+    else MBIR_MODE(false, false);
+#undef MBIR_MODE
 }
 
 IcdConst make_icd_const(const Geom &g)
@@ -780,21 +1043,18 @@ IcdConst make_icd_const(const Geom &g)
     K.tf = (float)g.time_filter;
     K.q = (float)g.q;
     K.qmp = (float)(g.q - g.p);
-    K.ssq = (float)g.sigma_s_q;
-    K.ssqp = (float)g.sigma_s_q_p;
-    K.stq = (float)g.sigma_t_q;
-    K.stqp = (float)g.sigma_t_q_p;
     K.issq = (float)(1.0 / g.sigma_s_q);
     K.issqp = (float)(1.0 / g.sigma_s_q_p);
     K.istq = (float)(1.0 / g.sigma_t_q);
     K.istqp = (float)(1.0 / g.sigma_t_q_p);
     K.cs = (float)g.c_s;
     K.ct = (float)g.c_t;
-    K.bs0 = (float)(g.q / (g.sigma_s_q * g.c_s));
-    K.bt0 = (float)(g.q / (g.sigma_t_q * g.c_t));
+    K.qocs = (float)(g.q / g.c_s);
+    K.qoct = (float)(g.q / g.c_t);
     K.alpha = (float)g.alpha;
     K.dt = (float)g.delta_t;
     K.huber_T = (float)g.huber_T;
+    K.huber_T2 = (float)(g.huber_T * g.huber_T * (1.0 - 1e-5));
     K.huber_delta = (float)g.huber_delta;
     K.huber = g.huber;
     return K;
@@ -805,26 +1065,14 @@ void launch_icd_phase(const Geom &g, const IcdLaunch &L, const uint32_t *d_table
                       IcdStats *d_stats, unsigned int *d_queue, cudaStream_t st)
 {
     const IcdConst K = make_icd_const(g);
-#define MBIR_LAUNCH(KW, U, VEC) \
-    launch_kw<KW, U, VEC>(g, L, K, d_table, d_view_first, d_mask, d_x, d_err, d_w, d_mag, d_stats, d_queue, st)
-    const int kw = g.rec_words / 4;
     const bool v4 = g.N_t % 4 == 0;
-    if (kw == 1) {
-        if (L.unroll >= 2) {
-            if (v4) MBIR_LAUNCH(1, 2, 4);
-            else MBIR_LAUNCH(1, 2, 2);
-        } else {
-            if (v4) MBIR_LAUNCH(1, 1, 4);
-            else MBIR_LAUNCH(1, 1, 2);
-        }
-    } else if (kw == 2) {
-        if (v4) MBIR_LAUNCH(2, 1, 4);
-        else MBIR_LAUNCH(2, 1, 2);
-    } else {
-        if (v4) MBIR_LAUNCH(3, 1, 4);
-        else MBIR_LAUNCH(3, 1, 2);
-    }
-#undef MBIR_LAUNCH
+    // entries in flight: 8, or 4 where no view group has more (one view each: a
+    // batch is then mostly filling), or as the caller asks
+    const int gstride = L.warps * (32 / icd_lanes_per_row(g.N_t, v4 ? 4 : 2));
+    const int most = (g.max_views + gstride - 1) / gstride * g.kmax;
+    const bool b8 = L.unroll > 0 ? L.unroll >= 2 : most > 4;
+    const auto launch = v4 ? (b8 ? launch_vec<4, 8> : launch_vec<4, 4>) : (b8 ? launch_vec<2, 8> : launch_vec<2, 4>);
+    launch(g, L, K, d_table, d_view_first, d_mask, d_x, d_err, d_w, d_mag, d_stats, d_queue, st);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -835,16 +1083,26 @@ void launch_icd_phase(const Geom &g, const IcdLaunch &L, const uint32_t *d_table
 // CTA keeps the descriptor of its current problem in shared memory and
 // reloads it when its next item belongs to another problem. Problems of one
 // launch share the record width and the detector-row vector width (template
-// parameters).
-template <int KW, int kUnroll, int VEC>
+// parameter).
+//
+// 64 registers, four entries in flight, entry lists unpacked from global memory:
+// eight CTAs of four warps stay on an SM, as many super-voxels in flight as the
+// convergence bound allows. That number is part of the method here: updates that
+// run at once act as extra over-relaxation, which speeds the slow modes up until
+// it diverges. The staged sweep with its tile is faster per iteration (8.0 against
+// 10.6 ms on 12 problems, 16.1 before) but keeps only three CTAs on an SM, and a
+// 256 x 256 x 8 problem of 129 views was then at twice the cost after 16 iterations.
+template <int VEC>
 __global__ void __launch_bounds__(kMaxWarps * 32, 4) icd_batch_kernel(const BatchDesc *__restrict__ descs,
                                                                       const int2 *__restrict__ item_map, int total,
                                                                       int phase, unsigned int *__restrict__ queue)
 {
     __shared__ IcdSmem S;
     __shared__ __align__(16) BatchDesc P;
+    extern __shared__ __align__(16) uint32_t s_dyn[];
     int cur = -1;
     IcdCount cnt{};
+    init_copies(S);
     for (;;) {
         __syncthreads();
         if (threadIdx.x == 0) S.item = (int)atomicAdd(queue, 1u);
@@ -870,8 +1128,8 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 4) icd_batch_kernel(const Batc
         const int sx = K * (rem % hx) + color % K;
         const int sy = K * (rem / hx) + color / K;
         if (sx >= P.L.n_sv_x || sy >= P.L.n_sv_y) continue;
-        icd_update_sv<KW, kUnroll, VEC, false, 2>(P.g, P.L, P.K, P.table, P.view_first, P.mask, P.x, P.err, P.w, P.mag,
-                                               f, sx, sy, S, cnt, nullptr, 0);
+        icd_update_sv<VEC, false, false, 2, 4>(P.g, P.L, P.K, P.table, P.view_first, P.mask, P.x, P.err, P.w, P.mag, f, sx, sy,
+                                               S, cnt, s_dyn);
     }
     if (cur >= 0) flush_counts(cnt, P.stats);
 }
@@ -900,30 +1158,23 @@ __global__ void batch_end_iteration(BatchDesc *descs, int n)
     if (descs[i].L.iter > 1 && pct < descs[i].convg_thresh) descs[i].active = 0;
 }
 
-int batch_grid(int vec, int warps)
+void batch_plan(const Geom &g, IcdLaunch &L, int vec) { icd_plan_shared(g, L, vec, 4, ICD_PLAIN); }
+
+int batch_grid(int vec, int warps, int smem)
 {
     int dev = 0, sms = 148, per_sm = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (vec == 4) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, icd_batch_kernel<1, 2, 4>, warps * 32, 0);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, icd_batch_kernel<1, 2, 2>, warps * 32, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, vec == 4 ? icd_batch_kernel<4> : icd_batch_kernel<2>, warps * 32,
+                                                  smem);
     return sms * (per_sm > 0 ? per_sm : 1);
 }
 
-void launch_icd_batch(int vec, int warps, int grid, const BatchDesc *d_descs, const int2 *d_item_map, int total,
+void launch_icd_batch(int vec, int warps, int grid, int smem, const BatchDesc *d_descs, const int2 *d_item_map, int total,
                       int phase, unsigned int *d_queue, cudaStream_t st)
 {
-    if (vec == 4) icd_batch_kernel<1, 2, 4><<<grid, warps * 32, 0, st>>>(d_descs, d_item_map, total, phase, d_queue);
-    else icd_batch_kernel<1, 2, 2><<<grid, warps * 32, 0, st>>>(d_descs, d_item_map, total, phase, d_queue);
-}
-
-int icd_grid(int warps)
-{
-    int dev = 0, sms = 148, per_sm = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, icd_phase_kernel<1, 2, 4, false, 0>, warps * 32, 0);
-    return sms * (per_sm > 0 ? per_sm : 1);
+    if (vec == 4) icd_batch_kernel<4><<<grid, warps * 32, smem, st>>>(d_descs, d_item_map, total, phase, d_queue);
+    else icd_batch_kernel<2><<<grid, warps * 32, smem, st>>>(d_descs, d_item_map, total, phase, d_queue);
 }
 
 void launch_batch_begin(BatchDesc *d_descs, int n, cudaStream_t st)

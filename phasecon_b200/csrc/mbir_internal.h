@@ -122,7 +122,7 @@ struct IcdLaunch {
     int phase;            // 0..3
     int iter;             // 1-based iteration (zero-skipping starts at 2)
     int zero_skipping;
-    int unroll;           // views in flight per lane (1, 2, 4); the launcher caps it by record width
+    int unroll;           // entries in flight per lane: 0 by rule, 1 four, 2 and more eight
     uint64_t seed;
     const uint8_t *sel;   // [N_time][N_y][N_x] columns this sweep may visit (with the mask); null = all
     int perm;             // queue order inside a frame: SV slot = (queue index * perm) mod slots
@@ -135,7 +135,12 @@ struct IcdLaunch {
     // null = every SV slot of the phase's colour in every frame
     const uint32_t *items;
     const int *n_items;
+    // shared memory of a CTA, set by the launcher (icd_plan_shared): words of a
+    // record buffer, slots of a view group's entry list, words of all lists, views
+    // of one block of lists, bytes in all
+    int stage_words, list_cap, list_words, block_views, shared_bytes;
 };
+
 
 // SV slots of one colour per frame and the items (all frames) of one phase.
 inline int sv_slots(int N_x, int N_y, int sv, int K)
@@ -172,9 +177,10 @@ struct IcdStats {  // device accumulators
 struct IcdConst {
     float sf[27];
     float tf;
-    float q, qmp, ssq, ssqp, stq, stqp, cs, ct, bs0, bt0, alpha, dt;
-    float issq, issqp, istq, istqp;  // reciprocals of ssq, ssqp, stq, stqp
-    float huber_T, huber_delta;
+    float q, qmp, cs, ct, alpha, dt;
+    float issq, issqp, istq, istqp;  // reciprocals of the scale powers sigma^q, sigma^(q-p) (space, time)
+    float qocs, qoct;                // q / c: the surrogate weight at a zero difference times sigma^q
+    float huber_T, huber_T2, huber_delta;  // T2: T^2 less a margin for rounding
     int huber;
 };
 IcdConst make_icd_const(const Geom &g);
@@ -203,11 +209,12 @@ struct __align__(16) BatchDesc {
     int active;                        // 0 once converged: its items are skipped
     int iters_done;
 };
-int batch_grid(int vec, int warps);
-void launch_icd_batch(int vec, int warps, int grid, const BatchDesc *d_descs, const int2 *d_item_map, int total,
+// Shared-memory plan of one problem of a batched launch (fills L's fields),
+// the persistent grid, the launch.
+void batch_plan(const Geom &g, IcdLaunch &L, int vec);
+int batch_grid(int vec, int warps, int smem);
+void launch_icd_batch(int vec, int warps, int grid, int smem, const BatchDesc *d_descs, const int2 *d_item_map, int total,
                       int phase, unsigned int *d_queue, cudaStream_t st);
-// persistent grid of the one-problem sweep kernel at `warps` warps per CTA
-int icd_grid(int warps);
 // Stability of concurrent super-voxel updates: CTAs update different columns
 // at the same time, and columns of one frame on a common ray couple like a
 // Jacobi step, more strongly the closer they are. Same-colour SVs are K sv

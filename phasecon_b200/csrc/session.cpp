@@ -218,14 +218,40 @@ int Session::init(const mbirgpu_problem *pb, const mbirgpu_options *o, int mult_
 // Default schedule, a function of the problem's shape only (autotune = 0):
 // 4 x 4 super-voxels in K = 2 colours (the 4-D workload's measured best,
 // and the concurrency cap sv_max_concurrent keeps it convergent on any
-// frame size), 4 warps per column when a frame has at least 64 views to
-// split over them, else 2. Fields the user fixed are kept.
+// frame size). Warps per column: 2 where more than four SVs per SM may be in
+// flight (4-D workload: eight CTAs of two warps fit on an SM, so all 1,024 SVs the
+// bound allows run at once, as fast as four CTAs of four warps, 5.1 ms a sweep; but
+// the number at once is part of the convergence, and with 592 the cost after 13
+// iterations was 7e-5 higher) or a frame has fewer than 64 views to split over
+// more, else 4; where the SVs leave SMs
+// idle (small images: at most one SV per SM), the length of a column's chain is
+// all that counts: 4, or 8 when the column's entries give a lane of one warp more
+// than 64 (sweep of a 100 x 100 x 38 Huber problem, 75 views a frame: 4.2 ms
+// with 4 warps, 2.9 with 8; 64 x 64 x 8, 90 views, 13 entries: 0.52 both ways).
+// Fields the user fixed are kept.
+constexpr long long kSms = 148;
+
+// super-voxels that one colour phase updates at once
+long long Session::in_flight(int sv_, int colors_) const
+{
+    const Geom &g = hs.g;
+    return std::min((long long)g.N_time * sv_slots(g.N_x, g.N_y, sv_, colors_),
+                    sv_max_concurrent(g.N_x, g.N_y, g.N_time, sv_, colors_));
+}
+
 void Session::choose_schedule()
 {
     const Geom &g = hs.g;
     sv = opt.sv_size > 0 ? std::min(opt.sv_size, 16) : 4;
     colors = opt.sv_colors > 0 ? opt.sv_colors : 2;
-    warps = opt.cta_warps > 0 ? std::min(opt.cta_warps, 8) : (g.max_views >= 64 ? 4 : 2);
+    if (opt.cta_warps > 0) {
+        warps = std::min(opt.cta_warps, 8);
+    } else if (in_flight(sv, colors) > kSms) {
+        warps = g.max_views >= 64 && in_flight(sv, colors) <= 4 * kSms ? 4 : 2;
+    } else {
+        const double lane_entries = 2.27 * g.max_views * g.N_t / (32.0 * (g.N_t % 4 == 0 ? 4 : 2));
+        warps = lane_entries > 64 ? 8 : 4;
+    }
     sync_nh_schedule();
 }
 
@@ -242,16 +268,18 @@ void Session::choose_schedule()
 // different schedules and end on (equally converged) different images.
 
 // Schedule of the non-homogeneous passes: the user's, else the full sweep's
-// super-voxels and colours with twice its warps per column (up to 8). Those
-// passes are bound by chains of column updates inside the few super-voxels
-// that hold many selected columns, so a shorter time per column pays more
-// than the occupancy the wider CTAs cost (4-D workload: 18.6 ms per
-// iteration with 8 warps against 20.6 ms with 4).
+// super-voxels and colours, with 4 warps per column where the SVs in flight fill
+// the GPU (4-D workload: 12.1 ms per iteration with 4, 13.5 with 2, 14.6 with 8)
+// and twice the sweep's, up to 8, where they do not (chains of column updates
+// inside the few super-voxels that hold many selected columns: 100 x 100 x 38
+// Huber problem, 10.1 ms with 8 against 12.6 with 4).
 void Session::sync_nh_schedule()
 {
     nh_sv = opt.nh_sv_size > 0 ? std::min(opt.nh_sv_size, 16) : sv;
     nh_colors = opt.nh_sv_colors > 0 ? opt.nh_sv_colors : colors;
-    nh_warps = opt.nh_cta_warps > 0 ? std::min(opt.nh_cta_warps, 8) : std::min(8, 2 * warps);
+    nh_warps = opt.nh_cta_warps > 0 ? std::min(opt.nh_cta_warps, 8)
+               : in_flight(nh_sv, nh_colors) > 2 * kSms ? 4
+                                                        : std::min(8, 2 * warps);
 }
 
 int Session::autotune()
@@ -375,7 +403,7 @@ int Session::enqueue_iteration(int iter, bool graph_mode, int *launches_out)
     L.iter = iter;
     L.iter_dev = graph_mode ? d_iter : nullptr;
     L.zero_skipping = opt.zero_skipping;
-    L.unroll = opt.icd_unroll > 0 ? opt.icd_unroll : 4;
+    L.unroll = opt.icd_unroll;
     L.seed = opt.seed;
     L.colors_k = colors;
     L.perm = spread_multiplier(sv_slots(g.N_x, g.N_y, sv, colors));

@@ -70,6 +70,7 @@ struct Session {
     ~Session();
     int init(const mbirgpu_problem *pb, const mbirgpu_options *o, int mult_xy, int mult_z, void *stream);
     void choose_schedule();
+    long long in_flight(int sv_, int colors_) const;
     int autotune();
     void sync_nh_schedule();
     struct TuneEntry {
