@@ -7,7 +7,7 @@
 // float like filtMagUpdateMap); the threshold is the (N - k)-th smallest
 // filtered value over all N = N_y N_x columns (RandomizedSelect's order
 // statistic), found here by an exact 4-digit radix select on the float bit
-// patterns (non-negative floats order like their bits) spread over many CTAs
+// patterns (non-negative floats order like their bits) by a cluster of CTAs
 // per frame; the selected columns
 // are those strictly above it -- the k largest -- that lie inside the mask
 // (the reference also picks unmasked columns near the edge but its update
@@ -26,83 +26,52 @@ __constant__ double c_hamming[5][5] = {{0.0064, 0.0432, 0.0800, 0.0432, 0.0064},
                                        {0.0432, 0.2916, 0.5400, 0.2916, 0.0432},
                                        {0.0064, 0.0432, 0.0800, 0.0432, 0.0064}};
 
-__global__ void vsc_filter_kernel(int n_frames, int NY, int NX, const float *__restrict__ mag,
-                                  float *__restrict__ filt)
+// filtered update magnitude of column (j, k): the reference's 5x5 window in its
+// (p, q) order, FP64 without contraction, as the host
+__device__ __forceinline__ float vsc_filter(const float *__restrict__ m, int j, int k, int NY, int NX)
 {
-    const int nxy = NX * NY;
-    const long long n = (long long)n_frames * nxy;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int f = (int)(i / nxy), c = (int)(i - (long long)f * nxy);
-        const int j = c / NX, k = c - j * NX;
-        const float *m = mag + (size_t)f * nxy;
-        double acc = 0.0;
-        for (int p = -2; p <= 2; p++) {
-            const int jj = j + p;
-            if (jj < 0 || jj >= NY) continue;
-            for (int q = -2; q <= 2; q++) {
-                const int kk = k + q;
-                if (kk < 0 || kk >= NX) continue;
-                acc = __dadd_rn(acc, __dmul_rn(c_hamming[p + 2][q + 2], (double)m[jj * NX + kk]));  // no contraction, as the host
-            }
-        }
-        filt[i] = (float)acc;
-    }
-}
-
-// number of selected columns of every (frame, SV); histogram per (phase, count)
-__global__ void nh_count_kernel(int n_frames, int NY, int NX, int sv, int K, const uint8_t *__restrict__ sel,
-                                int *__restrict__ svcount, int *__restrict__ hist)
-{
-    const int nsx = (NX + sv - 1) / sv, nsy = (NY + sv - 1) / sv, maxc = sv * sv;
-    const long long n = (long long)n_frames * nsx * nsy;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int f = (int)(i / ((long long)nsx * nsy));
-        const int r = (int)(i - (long long)f * nsx * nsy), sy = r / nsx, sx = r - sy * nsx;
-        const uint8_t *s = sel + (size_t)f * NX * NY;
-        int cnt = 0;
-        for (int a = 0; a < sv; a++) {
-            const int j = sy * sv + a;
-            if (j >= NY) break;
-            for (int b = 0; b < sv; b++) {
-                const int k = sx * sv + b;
-                if (k < NX) cnt += s[j * NX + k] != 0;
-            }
-        }
-        svcount[i] = cnt;
-        if (cnt) {
-            const int color = (sy % K) * K + sx % K;
-            const int phase = ((color - f) % (K * K) + K * K) % (K * K);
-            atomicAdd(&hist[phase * (maxc + 1) + cnt], 1);
+    double acc = 0.0;
+#pragma unroll
+    for (int p = -2; p <= 2; p++) {
+        const int jj = j + p;
+        if (jj < 0 || jj >= NY) continue;
+#pragma unroll
+        for (int q = -2; q <= 2; q++) {
+            const int kk = k + q;
+            if (kk < 0 || kk >= NX) continue;
+            acc = __dadd_rn(acc, __dmul_rn(c_hamming[p + 2][q + 2], (double)m[jj * NX + kk]));
         }
     }
-}
-
-// per phase: bucket offsets, counts descending; the phase's total
-__global__ void nh_offsets_kernel(int phases, int maxc, const int *__restrict__ hist, int *__restrict__ off,
-                                  int *__restrict__ n_items)
-{
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= phases) return;
-    int o = 0;
-    for (int c = maxc; c >= 1; c--) {
-        off[p * (maxc + 1) + c] = o;
-        o += hist[p * (maxc + 1) + c];
-    }
-    n_items[p] = o;
+    return (float)acc;
 }
 
 // walk each phase's SVs in the sweep's own queue order (frames fastest, spread
 // slots) and append the non-empty ones to their count's bucket
-__global__ void nh_scatter_kernel(int n_frames, int NY, int NX, int sv, int K, int perm, int per_phase,
-                                  const int *__restrict__ svcount, const int *__restrict__ off,
-                                  int *__restrict__ cursor, uint32_t *__restrict__ items)
+__global__ void __launch_bounds__(256) nh_scatter_kernel(int n_frames, int NY, int NX, int sv, int K, int perm, int per_phase,
+                                                         const int *__restrict__ svcount, const int *__restrict__ hist,
+                                                         int *__restrict__ cursor, uint32_t *__restrict__ items,
+                                                         int *__restrict__ n_items)
 {
+    // the bucket of c columns starts after the buckets of more: every CTA adds
+    // up its phase's histogram (blockIdx.y: the phase)
+    __shared__ int s_off[257];
+    const int p = blockIdx.y;
     const int nsx = (NX + sv - 1) / sv, nsy = (NY + sv - 1) / sv, maxc = sv * sv, KK = K * K;
+    for (int c = threadIdx.x; c <= maxc; c += blockDim.x) s_off[c] = hist[p * (maxc + 1) + c];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        int o = 0;
+        for (int c = maxc; c >= 1; c--) {
+            const int h = s_off[c];
+            s_off[c] = o;
+            o += h;
+        }
+        if (blockIdx.x == 0) n_items[p] = o;
+    }
+    __syncthreads();
     const int hx = (nsx + K - 1) / K, slots = hx * ((nsy + K - 1) / K);
-    const long long n = (long long)KK * n_frames * slots;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int p = (int)(i / ((long long)n_frames * slots));
-        const int q = (int)(i - (long long)p * n_frames * slots);
+    const int n = n_frames * slots;
+    for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += gridDim.x * blockDim.x) {
         const int f = q % n_frames;
         const int rem = (int)((long long)(q / n_frames) * perm % slots);
         const int color = (p + f) % KK;
@@ -111,84 +80,125 @@ __global__ void nh_scatter_kernel(int n_frames, int NY, int NX, int sv, int K, i
         const int cnt = svcount[((size_t)f * nsy + sy) * nsx + sx];
         if (!cnt) continue;
         const int pos = atomicAdd(&cursor[p * (maxc + 1) + cnt], 1);
-        items[(size_t)p * per_phase + off[p * (maxc + 1) + cnt] + pos] =
-            ((uint32_t)f << 22) | ((uint32_t)sy << 11) | (uint32_t)sx;
+        items[(size_t)p * per_phase + s_off[cnt] + pos] = ((uint32_t)f << 22) | ((uint32_t)sy << 11) | (uint32_t)sx;
     }
 }
 
-// The order statistic by radix select over the float bit patterns, spread
-// over many CTAs per frame: per 8-bit digit (most significant first) a
-// histogram kernel over all keys that match the prefix so far, then a
-// one-warp-per-frame kernel that picks the digit holding the rank (the
-// (k+1)-th largest key, the threshold); state[f] = {prefix, prefix mask,
-// remaining rank, found}. sel = mask && key > threshold: the k largest.
-struct NhSelState {
-    unsigned int prefix, pmask;
-    int rank, found;
-};
+// The selection of one pass, one cluster of kSelCtas CTAs per frame: the filtered
+// map; its threshold, the (k + 1)-th largest value, by radix select over the float
+// bit patterns, eight bits a round (each CTA's histogram of the keys that match
+// the digits so far in its shared memory, added up over the cluster through
+// distributed shared memory, so every CTA finds the same digit); sel = mask && key
+// > threshold; and, when svcount is given, the selected columns of every
+// super-voxel with a histogram per (phase, count). One launch: as eleven (filter,
+// four histogram / pick pairs, ...) a pass's selection took about 65 us, most of it
+// launches and one thread scanning 256 bins.
+constexpr int kSelCtas = 8, kSelThreads = 1024;
+constexpr int kSelKeys = 8;  // keys a thread keeps in registers (images up to 256 x 256 entirely)
 
-__global__ void nh_sel_init_kernel(int n_frames, int k, NhSelState *__restrict__ state, unsigned int *__restrict__ ghist)
+__device__ __forceinline__ void cluster_sync()
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n_frames) state[i] = NhSelState{0u, 0u, k + 1, 1};
-    for (int b = i; b < n_frames * 256; b += gridDim.x * blockDim.x) ghist[b] = 0u;
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ unsigned remote_load(const unsigned *p, unsigned rank)
+{
+    unsigned a, v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
 }
 
-__global__ void nh_sel_hist_kernel(int nxy, int shift, const float *__restrict__ filt,
-                                   const NhSelState *__restrict__ state, unsigned int *__restrict__ ghist)
+__global__ void __cluster_dims__(kSelCtas, 1, 1) __launch_bounds__(kSelThreads)
+    nh_select_kernel(int NY, int NX, int k, const float *__restrict__ mag, const uint8_t *__restrict__ mask,
+                     float *__restrict__ filt, uint8_t *__restrict__ sel, int sv, int K, int *__restrict__ svcount,
+                     int *__restrict__ hist_out)
 {
-    __shared__ unsigned int hist[256];
-    const int f = blockIdx.y;
-    const NhSelState st = state[f];
-    if (!st.found) return;  // uniform: this frame's selection is settled
-    for (int b = threadIdx.x; b < 256; b += blockDim.x) hist[b] = 0u;
-    __syncthreads();
-    const unsigned int *key = reinterpret_cast<const unsigned int *>(filt + (size_t)f * nxy);
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nxy; i += gridDim.x * blockDim.x) {
-        const unsigned int u = key[i];
-        if ((u & st.pmask) == st.prefix) atomicAdd(&hist[(u >> shift) & 255u], 1u);
+    __shared__ unsigned s_hist[256], s_sum[256];
+    __shared__ unsigned s_digit, s_above;
+    const int f = blockIdx.x / kSelCtas, rank = blockIdx.x % kSelCtas;
+    const int nxy = NX * NY, first = rank * kSelThreads + threadIdx.x, stride = kSelCtas * kSelThreads;
+    const float *m = mag + (size_t)f * nxy;
+    float *fm = filt + (size_t)f * nxy;
+    uint8_t *sm = sel + (size_t)f * nxy;
+    unsigned key[kSelKeys];
+    const int rest = first + kSelKeys * stride;  // columns past those: filtered into fm, read back by the same thread
+#pragma unroll
+    for (int i = 0; i < kSelKeys; i++) {
+        const int c = first + i * stride;
+        key[i] = c < nxy ? __float_as_uint(vsc_filter(m, c / NX, c % NX, NY, NX)) : 0u;
     }
-    __syncthreads();
-    for (int b = threadIdx.x; b < 256; b += blockDim.x)
-        if (hist[b]) atomicAdd(&ghist[f * 256 + b], hist[b]);
-}
-
-// one warp per frame: the digit whose cumulative count from the top reaches
-// the rank; clears the histogram for the next digit
-__global__ void nh_sel_pick_kernel(int shift, NhSelState *__restrict__ state, unsigned int *__restrict__ ghist)
-{
-    const int f = blockIdx.x, lane = threadIdx.x;
-    NhSelState st = state[f];
-    unsigned int *h = ghist + f * 256;
-    if (st.found && lane == 0) {
-        int cum = 0, b = 255;
-        for (; b >= 0; b--) {
-            if (cum + (int)h[b] >= st.rank) break;
-            cum += (int)h[b];
+    for (int c = rest; c < nxy; c += stride) fm[c] = vsc_filter(m, c / NX, c % NX, NY, NX);
+    unsigned prefix = 0, pmask = 0, need = (unsigned)k + 1;
+    bool found = true;
+    for (int shift = 24; shift >= 0 && found; shift -= 8) {  // uniform over the cluster
+        for (int b = threadIdx.x; b < 256; b += kSelThreads) s_hist[b] = 0u;
+        __syncthreads();
+        auto count = [&](unsigned u) {
+            if ((u & pmask) == prefix) atomicAdd(&s_hist[(u >> shift) & 255u], 1u);
+        };
+#pragma unroll
+        for (int i = 0; i < kSelKeys; i++)
+            if (first + i * stride < nxy) count(key[i]);
+        for (int c = rest; c < nxy; c += stride) count(__float_as_uint(fm[c]));
+        cluster_sync();
+        if (threadIdx.x < 256) {
+            unsigned t = 0;
+            for (unsigned r = 0; r < kSelCtas; r++) t += remote_load(&s_hist[threadIdx.x], r);
+            s_sum[threadIdx.x] = t;
         }
-        if (b < 0) {  // fewer than k + 1 keys: every key is above the threshold
-            st.found = 0;
-        } else {
-            st.prefix |= (unsigned int)b << shift;
-            st.pmask |= 0xFFu << shift;
-            st.rank -= cum;
+        __syncthreads();
+        // the digit at which the count from the top reaches the rank: lane l of warp 0
+        // holds digits 255 - 8 l .. 248 - 8 l
+        if (threadIdx.x < 32) {
+            unsigned h[8], t = 0;
+#pragma unroll
+            for (int i = 0; i < 8; i++) t += h[i] = s_sum[255 - 8 * threadIdx.x - i];
+            unsigned incl = t;
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned up = __shfl_up_sync(0xffffffffu, incl, o);
+                if (threadIdx.x >= o) incl += up;
+            }
+            const unsigned any = __ballot_sync(0xffffffffu, incl >= need);
+            if (any == 0) {
+                if (threadIdx.x == 0) s_digit = 256u;  // fewer keys than the rank: all are above the threshold
+            } else if ((int)threadIdx.x == __ffs(any) - 1) {
+                unsigned cum = incl - t;
+                int i = 0;
+                while (cum + h[i] < need) cum += h[i++];
+                s_digit = 255u - 8u * threadIdx.x - (unsigned)i;
+                s_above = cum;
+            }
         }
-        state[f] = st;
+        __syncthreads();
+        found = s_digit < 256u;
+        if (found) {
+            prefix |= s_digit << shift;
+            pmask |= 0xFFu << shift;
+            need -= s_above;
+        }
+        cluster_sync();  // every CTA has read this round's histograms
     }
-    __syncwarp();
-    for (int b = lane; b < 256; b += 32) h[b] = 0u;
-}
-
-__global__ void nh_sel_final_kernel(int n_frames, int nxy, int k, const float *__restrict__ filt,
-                                    const uint8_t *__restrict__ mask, const NhSelState *__restrict__ state,
-                                    uint8_t *__restrict__ sel)
-{
-    const long long n = (long long)n_frames * nxy;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        const int f = (int)(i / nxy), c = (int)(i - (long long)f * nxy);
-        const unsigned int u = reinterpret_cast<const unsigned int *>(filt)[i];
-        const NhSelState st = state[f];
-        sel[i] = (uint8_t)(k > 0 && mask[c] && (!st.found || u > st.prefix));
+#pragma unroll
+    for (int i = 0; i < kSelKeys; i++) {
+        const int c = first + i * stride;
+        if (c < nxy) sm[c] = (uint8_t)(k > 0 && mask[c] && (!found || key[i] > prefix));
+    }
+    for (int c = rest; c < nxy; c += stride)
+        sm[c] = (uint8_t)(k > 0 && mask[c] && (!found || __float_as_uint(fm[c]) > prefix));
+    if (!svcount) return;
+    cluster_sync();  // the frame's selection is complete
+    const int nsx = (NX + sv - 1) / sv, nsy = (NY + sv - 1) / sv, maxc = sv * sv;
+    for (int i = first; i < nsx * nsy; i += stride) {
+        const int sy = i / nsx, sx = i - sy * nsx;
+        int cnt = 0;
+        for (int a = 0; a < sv && sy * sv + a < NY; a++)
+            for (int b = 0; b < sv && sx * sv + b < NX; b++) cnt += __ldcg(sm + (sy * sv + a) * NX + sx * sv + b) != 0;
+        svcount[(size_t)f * nsx * nsy + i] = cnt;
+        if (cnt) {
+            const int color = (sy % K) * K + sx % K;
+            const int phase = ((color - f) % (K * K) + K * K) % (K * K);
+            atomicAdd(&hist_out[phase * (maxc + 1) + cnt], 1);
+        }
     }
 }
 
@@ -199,10 +209,11 @@ int nh_items_per_phase(int n_frames, int N_y, int N_x, int sv, int K)
     return n_frames * sv_slots(N_x, N_y, sv, K);
 }
 
+// [svcount | hist | cursor]
 size_t nh_items_scratch_ints(int n_frames, int N_y, int N_x, int sv, int K)
 {
     const size_t nsv = (size_t)((N_x + sv - 1) / sv) * ((N_y + sv - 1) / sv);
-    return (size_t)n_frames * nsv + 3 * (size_t)K * K * (sv * sv + 1);
+    return (size_t)n_frames * nsv + 2 * (size_t)K * K * (sv * sv + 1);
 }
 
 bool nh_items_supported(int n_frames, int N_y, int N_x, int sv)
@@ -210,47 +221,27 @@ bool nh_items_supported(int n_frames, int N_y, int N_x, int sv)
     return n_frames <= 1024 && (N_x + sv - 1) / sv <= 2048 && (N_y + sv - 1) / sv <= 2048;
 }
 
-void launch_nh_items(int n_frames, int N_y, int N_x, int sv, int K, const uint8_t *d_sel, uint32_t *d_items,
-                     int *d_n_items, int *d_scratch, cudaStream_t st)
+void launch_nh_select(int n_frames, int N_y, int N_x, const float *d_mag, const uint8_t *d_mask, int k,
+                      float *d_filt, uint8_t *d_sel, cudaStream_t st)
+{
+    nh_select_kernel<<<kSelCtas * n_frames, kSelThreads, 0, st>>>(N_y, N_x, k, d_mag, d_mask, d_filt, d_sel, 1, 1, nullptr,
+                                                                 nullptr);
+}
+
+void launch_nh_select_items(int n_frames, int N_y, int N_x, const float *d_mag, const uint8_t *d_mask, int k,
+                            float *d_filt, uint8_t *d_sel, int sv, int K, uint32_t *d_items, int *d_n_items,
+                            int *d_scratch, cudaStream_t st)
 {
     const int nsx = (N_x + sv - 1) / sv, nsy = (N_y + sv - 1) / sv, maxc = sv * sv, KK = K * K;
     const size_t nsv = (size_t)n_frames * nsx * nsy, hsz = (size_t)KK * (maxc + 1);
-    int *svcount = d_scratch, *hist = d_scratch + nsv, *off = hist + hsz, *cursor = off + hsz;
-    cudaMemsetAsync(hist, 0, hsz * sizeof(int), st);
-    cudaMemsetAsync(cursor, 0, hsz * sizeof(int), st);
-    const int blocks = (int)std::min<size_t>((nsv + 255) / 256, 148 * 8);
-    nh_count_kernel<<<blocks, 256, 0, st>>>(n_frames, N_y, N_x, sv, K, d_sel, svcount, hist);
-    nh_offsets_kernel<<<1, 32, 0, st>>>(KK, maxc, hist, off, d_n_items);
+    int *svcount = d_scratch, *hist = d_scratch + nsv, *cursor = hist + hsz;
+    cudaMemsetAsync(hist, 0, 2 * hsz * sizeof(int), st);
+    nh_select_kernel<<<kSelCtas * n_frames, kSelThreads, 0, st>>>(N_y, N_x, k, d_mag, d_mask, d_filt, d_sel, sv, K, svcount,
+                                                                 hist);
     const int per_phase = nh_items_per_phase(n_frames, N_y, N_x, sv, K);
-    const long long n = (long long)KK * per_phase;
-    const int sblocks = (int)std::min<long long>((n + 255) / 256, 148LL * 8);
-    nh_scatter_kernel<<<sblocks, 256, 0, st>>>(n_frames, N_y, N_x, sv, K,
-                                               spread_multiplier(sv_slots(N_x, N_y, sv, K)), per_phase, svcount, off,
-                                               cursor, d_items);
-}
-
-void launch_nh_select(int n_frames, int N_y, int N_x, const float *d_mag, const uint8_t *d_mask, int k,
-                      float *d_filt, uint8_t *d_sel, cudaStream_t st, void *d_sel_scratch)
-{
-    const int nxy = N_y * N_x;
-    const long long n = (long long)n_frames * nxy;
-    const int blocks = (int)std::min<long long>((n + 255) / 256, 148LL * 16);
-    vsc_filter_kernel<<<blocks, 256, 0, st>>>(n_frames, N_y, N_x, d_mag, d_filt);
-    NhSelState *state = reinterpret_cast<NhSelState *>(d_sel_scratch);
-    unsigned int *ghist = reinterpret_cast<unsigned int *>(state + n_frames);
-    nh_sel_init_kernel<<<(n_frames * 256 + 255) / 256, 256, 0, st>>>(n_frames, k, state, ghist);
-    // about 4 keys per thread: enough CTAs per frame to spread the reads over the GPU
-    const int per_frame = std::max(1, std::min(64, (nxy + 1023) / 1024));
-    for (int shift = 24; shift >= 0; shift -= 8) {
-        nh_sel_hist_kernel<<<dim3(per_frame, n_frames), 256, 0, st>>>(nxy, shift, d_filt, state, ghist);
-        nh_sel_pick_kernel<<<n_frames, 32, 0, st>>>(shift, state, ghist);
-    }
-    nh_sel_final_kernel<<<blocks, 256, 0, st>>>(n_frames, nxy, k, d_filt, d_mask, state, d_sel);
-}
-
-size_t nh_select_scratch_bytes(int n_frames)
-{
-    return (size_t)n_frames * (sizeof(NhSelState) + 256 * sizeof(unsigned int));
+    nh_scatter_kernel<<<dim3((per_phase + 255) / 256, KK), 256, 0, st>>>(
+        n_frames, N_y, N_x, sv, K, spread_multiplier(sv_slots(N_x, N_y, sv, K)), per_phase, svcount, hist, cursor, d_items,
+        d_n_items);
 }
 
 }  // namespace mbirgpu

@@ -65,7 +65,7 @@ Session::~Session()
 {
     void *ptrs[] = {d_y, d_w, d_err, d_x, d_tmp, d_table, d_Hr, d_cos, d_sin, d_views, d_view_first, d_view_frame,
                     d_mask, d_mag, d_stats, d_cost_partials, d_cost_out, d_flag, d_acc, d_queue, d_filt, d_sel,
-                    d_nh_items, d_nh_n, d_nh_scratch, d_nh_selstate, d_off, d_offx, d_onum, d_olam, d_ogamma,
+                    d_nh_items, d_nh_n, d_nh_scratch, d_off, d_offx, d_onum, d_olam, d_ogamma,
                     d_var};
     for (void *p : ptrs)
         if (p) cudaFree(p);
@@ -156,8 +156,7 @@ int Session::init(const mbirgpu_problem *pb, const mbirgpu_options *o, int mult_
                 nh_scratch_cap = std::max(nh_scratch_cap, nh_items_scratch_ints(g.N_time, g.N_y, g.N_x, sv, K));
         }
         if (dalloc(&d_nh_items, nh_items_cap, &acc) || dalloc(&d_nh_n, (size_t)kMaxPhases, &acc) ||
-            dalloc(&d_nh_scratch, nh_scratch_cap, &acc) ||
-            dalloc(&d_nh_selstate, (nh_select_scratch_bytes(g.N_time) + 7) / 8, &acc))
+            dalloc(&d_nh_scratch, nh_scratch_cap, &acc))
             return -1;
     }
 
@@ -430,7 +429,6 @@ int Session::enqueue_iteration(int iter, bool graph_mode, int *launches_out)
     if (nh > 0 && timing) CK(record(ev_pairs[1].first));
     for (int pass = 0; pass < nh; pass++) {
         const int k = (int)(masked_columns / std::max(1, g.N_time)) / kNhicdIterations;
-        launch_nh_select(g.N_time, g.N_y, g.N_x, d_mag, d_mask, k, d_filt, d_sel, st, d_nh_selstate);
         IcdLaunch Ln = L;
         Ln.sel = d_sel;
         Ln.seed = L.seed ^ (0x9E3779B97F4A7C15ull * (uint64_t)(pass + 1));
@@ -446,7 +444,11 @@ int Session::enqueue_iteration(int iter, bool graph_mode, int *launches_out)
         const bool lists = opt.nh_work_lists && nh_items_supported(g.N_time, g.N_y, g.N_x, nh_sv) &&
                            (size_t)nh_phases * per_phase <= nh_items_cap &&
                            nh_items_scratch_ints(g.N_time, g.N_y, g.N_x, nh_sv, nh_colors) <= nh_scratch_cap;
-        if (lists) launch_nh_items(g.N_time, g.N_y, g.N_x, nh_sv, nh_colors, d_sel, d_nh_items, d_nh_n, d_nh_scratch, st);
+        if (lists)
+            launch_nh_select_items(g.N_time, g.N_y, g.N_x, d_mag, d_mask, k, d_filt, d_sel, nh_sv, nh_colors, d_nh_items,
+                                   d_nh_n, d_nh_scratch, st);
+        else
+            launch_nh_select(g.N_time, g.N_y, g.N_x, d_mag, d_mask, k, d_filt, d_sel, st);
         for (int ph = 0; ph < nh_phases; ph++) {
             Ln.phase = ph;
             Ln.items = lists ? d_nh_items + (size_t)ph * per_phase : nullptr;
@@ -455,7 +457,7 @@ int Session::enqueue_iteration(int iter, bool graph_mode, int *launches_out)
                              d_queue + kMaxPhases * (pass + 1) + ph, st);
         }
         if (rings && update_offset()) return -1;
-        launches += nh_phases + 11 + (lists ? 3 : 0);  // filter + 10 select launches, 3 list launches
+        launches += nh_phases + 1 + (lists ? 1 : 0);  // the selection, the work lists
     }
     if (nh > 0 && timing) CK(record(ev_pairs[1].second));
     CK(cudaGetLastError());
@@ -1036,15 +1038,13 @@ int mbirgpu_session_nh_select(mbirgpu_session *sp, const float *mag, uint8_t *se
     const size_t n = (size_t)g.N_time * g.N_y * g.N_x;
     float *d_m = nullptr, *d_f = nullptr;
     uint8_t *d_s = nullptr;
-    void *d_scr = nullptr;
     cudaError_t e = cudaMalloc((void **)&d_m, n * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc((void **)&d_f, n * sizeof(float));
     if (e == cudaSuccess) e = cudaMalloc((void **)&d_s, n);
-    if (e == cudaSuccess) e = cudaMalloc(&d_scr, mbirgpu::nh_select_scratch_bytes(g.N_time));
     if (e == cudaSuccess) e = cudaMemcpyAsync(d_m, mag, n * sizeof(float), cudaMemcpyHostToDevice, s->st);
     if (e == cudaSuccess) {
         const int k = (int)(s->masked_columns / std::max(1, g.N_time)) / mbirgpu::kNhicdIterations;
-        mbirgpu::launch_nh_select(g.N_time, g.N_y, g.N_x, d_m, s->d_mask, k, d_f, d_s, s->st, d_scr);
+        mbirgpu::launch_nh_select(g.N_time, g.N_y, g.N_x, d_m, s->d_mask, k, d_f, d_s, s->st);
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaMemcpyAsync(sel, d_s, n, cudaMemcpyDeviceToHost, s->st);
@@ -1052,7 +1052,6 @@ int mbirgpu_session_nh_select(mbirgpu_session *sp, const float *mag, uint8_t *se
     cudaFree(d_m);
     cudaFree(d_f);
     cudaFree(d_s);
-    cudaFree(d_scr);
     if (e != cudaSuccess) return fail("NH-ICD selection failed: %s", cudaGetErrorString(e));
     return 0;
 }
