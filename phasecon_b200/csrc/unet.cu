@@ -34,14 +34,12 @@
 #include <vector>
 
 #include "../../include/mbirgpu.h"
+#include "conv_tc.h"
 #include "mbir_internal.h"
 
 namespace mbirgpu {
 
 int fail(const char *fmt, ...);
-int conv_tc_launch(const __nv_bfloat16 *in, int Kin, const __nv_bfloat16 *wt, __nv_bfloat16 *wtc, const float *bias,
-                   __nv_bfloat16 *out, int Nout, int d, int h, int w, int df, int relu, cudaStream_t st);
-int conv_tc_status(cudaStream_t st);
 
 namespace {
 
@@ -421,7 +419,7 @@ template <int NT>
 __host__ __device__ constexpr int wgrad_stage() { return kHalo * kGradPad + kTileVox * (NT + 8); }  // bf16 of one stage
 
 template <int NT>
-__global__ void __launch_bounds__(256) conv_wgrad_kernel(const bf16 *__restrict__ in, int Cin,
+__global__ void __launch_bounds__(256) conv_wgrad_kernel(const ConvIn in, int Cin,
                                                          const bf16 *__restrict__ gout, int Cout,
                                                          float *__restrict__ dw, float *__restrict__ db, int D, int H,
                                                          int W)
@@ -459,7 +457,7 @@ __global__ void __launch_bounds__(256) conv_wgrad_kernel(const bf16 *__restrict_
             const int hz = hv / (HY * HX), q = hv - hz * (HY * HX), hy = q / HX, hx = q - hy * HX;
             const int z = z0 + hz - 1, y = y0 + hy - 1, x = x0 + hx - 1;
             const bool ok = z >= 0 && z < D && y >= 0 && y < H && x >= 0 && x < W && c0 + 8 * half < Cin;
-            copy16(hs + hv * kGradPad + 8 * half, ok ? in + (((long long)z * H + y) * W + x) * Cin + c0 + 8 * half : in, ok);
+            copy16(hs + hv * kGradPad + 8 * half, ok ? in.piece(z, y, x, H, W, c0 + 8 * half) : in.a, ok);
         }
         for (int e = threadIdx.x; e < kTileVox * (NT / 8); e += 256) {
             const int tv = e / (NT / 8), p = e - tv * (NT / 8);
@@ -974,6 +972,8 @@ __global__ void copy_to_bf16_kernel(const float *__restrict__ p, long long n, bf
         pb[i] = __float2bfloat16(p[i]);
 }
 
+inline ConvIn plain(const bf16 *t, int channels) { return ConvIn{t, nullptr, channels, 0, 0}; }
+
 inline unsigned grid_for(long long n, int threads = 256)
 {
     return (unsigned)std::max<long long>(1, std::min<long long>((n + threads - 1) / threads, 148LL * 32));
@@ -992,7 +992,9 @@ struct UNet {
     size_t head_w = 0, head_b = 0, n_params = 0;
     float *d_p = nullptr, *d_g = nullptr, *d_m = nullptr, *d_v = nullptr;
     bf16 *d_pb = nullptr, *d_wt = nullptr;  // BF16 copy; flipped weights scratch
-    bf16 *d_wtc = nullptr;                   // weights re-laid for the tcgen05 kernel
+    bf16 *d_wtc = nullptr;                   // every convolution's weights re-laid for the tcgen05 kernel
+    std::vector<ConvTcWeights> tc;           // where each convolution's lie
+    ConvTcWeights *d_tc = nullptr;
     bool tensor_path = true;                 // tcgen05 convolutions where the shape allows
     bool conv_err = false;                   // a tcgen05 launch failed
     long long steps = 0;
@@ -1018,7 +1020,7 @@ struct UNet {
         free_acts();
         for (auto &b : spare) cudaFree(b.second);
         for (void *p : {(void *)d_p, (void *)d_g, (void *)d_m, (void *)d_v, (void *)d_pb, (void *)d_wt,
-                        (void *)d_wtc, (void *)d_loss})
+                        (void *)d_wtc, (void *)d_tc, (void *)d_loss})
             if (p) cudaFree(p);
     }
     // Activation blocks go back to a size-keyed pool instead of to the driver:
@@ -1034,9 +1036,19 @@ struct UNet {
     int init(int base, uint64_t seed);
     int ensure(int d, int h, int w, int frames = 1, bool grads = true);
     long long vox(int l) const { return (long long)(D >> l) * (H >> l) * (W >> l); }
-    void conv(int i, const bf16 *in, bf16 *o, int l, bool relu);
-    void conv_tiles(const bf16 *in, int Kin, const float *bias, bf16 *o, int Nout, int l, bool relu);
-    void conv_back(int i, const bf16 *in, const bf16 *o, bf16 *go, bf16 *gin, int l);
+    void conv(int i, const ConvIn &in, bf16 *o, int l, bool relu);
+    void conv_tiles(int i, bool grad, const ConvIn &in, int Kin, const float *bias, bf16 *o, int Nout, int l, bool relu);
+    // whether convolution i at level l reads a concatenated or upsampled input in
+    // place (else it is written out first)
+    bool in_place(int i, int l) const
+    {
+        return tensor_path && conv_tc_serves(convs[i].cin, convs[i].cout, D >> l, Df >> l);
+    }
+    ConvIn decoder_in(int i, int l, const bf16 *coarse) const;
+    ConvIn skip_in(int i, int l) const;
+    // the BF16 copy of the parameters has changed
+    void weights_changed() { conv_tc_weights(d_tc, (int)tc.size(), d_pb, d_wtc, st); }
+    void conv_back(int i, const ConvIn &in, const bf16 *o, bf16 *go, bf16 *gin, int l);
     int forward(const float *d_in);
     int backward(const float *d_target, double *loss);
     int step(float lr);
@@ -1086,13 +1098,22 @@ int UNet::init(int base, uint64_t seed)
     size_t wt = 0;
     for (auto &k : convs) wt = std::max(wt, (size_t)27 * k.cin * k.cout);
     if (e == cudaSuccess) e = cudaMalloc((void **)&d_wt, wt * sizeof(bf16));
-    if (e == cudaSuccess) e = cudaMalloc((void **)&d_wtc, wt * sizeof(bf16));
+    size_t relaid = 0;
+    for (auto &k : convs) {
+        const size_t n = (size_t)27 * k.cin * k.cout;
+        tc.push_back({k.cin, k.cout, conv_tc_split(k.cin, k.cout), conv_tc_split(k.cout, k.cin), k.w, relaid, relaid + n});
+        relaid += 2 * n;
+    }
+    if (e == cudaSuccess) e = cudaMalloc((void **)&d_wtc, relaid * sizeof(bf16));
+    if (e == cudaSuccess) e = cudaMalloc((void **)&d_tc, tc.size() * sizeof(ConvTcWeights));
+    if (e == cudaSuccess) e = cudaMemcpy(d_tc, tc.data(), tc.size() * sizeof(ConvTcWeights), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMalloc((void **)&d_loss, sizeof(double));
     if (e == cudaSuccess) e = cudaMemcpy(d_p, h.data(), n_params * sizeof(float), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(d_m, 0, n_params * sizeof(float));
     if (e == cudaSuccess) e = cudaMemset(d_v, 0, n_params * sizeof(float));
     if (e != cudaSuccess) return fail("U-Net allocation failed: %s", cudaGetErrorString(e));
     copy_to_bf16_kernel<<<grid_for((long long)n_params), 256, 0, st>>>(d_p, (long long)n_params, d_pb);
+    weights_changed();
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e == cudaSuccess)
@@ -1170,17 +1191,22 @@ int UNet::ensure(int d, int h, int w, int frames, bool grads)
     return 0;
 }
 
-// out = act(conv(in)) with weights in the tile layout (d_wt); Nout output channels.
-void UNet::conv_tiles(const bf16 *in, int Kin, const float *bias, bf16 *o, int Nout, int l, bool relu)
+// out = act(conv(in)) with convolution i's weights, or (grad) its data gradient;
+// Nout output channels.
+void UNet::conv_tiles(int i, bool grad, const ConvIn &cin_, int Kin, const float *bias, bf16 *o, int Nout, int l, bool relu)
 {
     const int d = D >> l, h = H >> l, w = W >> l, df = Df >> l;
     const unsigned tiles = (unsigned)(((d + FZ - 1) / FZ) * ((h + FY - 1) / FY) * ((w + FX - 1) / FX));
     const int r = relu ? 1 : 0;
     if (tensor_path) {
-        const int done = conv_tc_launch(in, Kin, d_wt, d_wtc, bias, o, Nout, d, h, w, df, r, st);
+        const int done = conv_tc_launch(cin_, Kin, d_wtc + (grad ? tc[i].out_grad : tc[i].out), bias, o, Nout, d, h, w, df, r,
+                                        st);
         if (done < 0) conv_err = true;
         if (done) return;
     }
+    const bf16 *in = cin_.a;  // the kernels below read one plain tensor (in_place)
+    const Conv &k = convs[i];
+    tile_weights_kernel<<<grid_for(27LL * k.cin * k.cout), 256, 0, st>>>(d_pb + k.w, k.cin, k.cout, grad ? 1 : 0, d_wt);
     if (Kin == 1) {
         dim3 grid(tiles, (unsigned)((Nout + 15) / 16));
         conv_first_kernel<16><<<grid, kFThreads, 0, st>>>(in, d_wt, bias, o, Nout, d, h, w, r, df);
@@ -1196,16 +1222,15 @@ void UNet::conv_tiles(const bf16 *in, int Kin, const float *bias, bf16 *o, int N
     }
 }
 
-void UNet::conv(int i, const bf16 *in, bf16 *o, int l, bool relu)
+void UNet::conv(int i, const ConvIn &in, bf16 *o, int l, bool relu)
 {
     const Conv &k = convs[i];
-    tile_weights_kernel<<<grid_for(27LL * k.cin * k.cout), 256, 0, st>>>(d_pb + k.w, k.cin, k.cout, 0, d_wt);
-    conv_tiles(in, k.cin, d_p + k.b, o, k.cout, l, relu);
+    conv_tiles(i, false, in, k.cin, d_p + k.b, o, k.cout, l, relu);
 }
 
 // o = relu(conv(in)); go: gradient w.r.t. o (overwritten by the ReLU mask);
 // gin (may be null): gradient w.r.t. in.
-void UNet::conv_back(int i, const bf16 *in, const bf16 *o, bf16 *go, bf16 *gin, int l)
+void UNet::conv_back(int i, const ConvIn &in, const bf16 *o, bf16 *go, bf16 *gin, int l)
 {
     const Conv &k = convs[i];
     const long long V = vox(l);
@@ -1218,7 +1243,7 @@ void UNet::conv_back(int i, const bf16 *in, const bf16 *o, bf16 *go, bf16 *gin, 
     const int nci = (k.cin + 15) / 16;
     if (k.cout % 8 == 0 && k.cin == 1) {
         const int nco = (k.cout + 15) / 16;
-        conv_wgrad_first_kernel<<<dim3((unsigned)std::min(tiles, 148 * 6), nco), 256, 0, st>>>(in, go, k.cout, d_g + k.w,
+        conv_wgrad_first_kernel<<<dim3((unsigned)std::min(tiles, 148 * 6), nco), 256, 0, st>>>(in.a, go, k.cout, d_g + k.w,
                                                                                               d_g + k.b, d, h, w);
     } else if (k.cout % 8 == 0 && k.cin % 8 == 0) {
         // four (NT = 16) or three CTAs to an SM, each adding its sums up once
@@ -1235,19 +1260,30 @@ void UNet::conv_back(int i, const bf16 *in, const bf16 *o, bf16 *go, bf16 *gin, 
         const unsigned gx = (unsigned)std::max(1, std::min(tiles, 4 * 148 / std::max(1, nci)));
         if (k.cout > 32) {
             dim3 grid(gx, (unsigned)nci, (unsigned)((k.cout + 63) / 64));
-            conv_wgrad_tile_kernel<64><<<grid, 256, 0, st>>>(in, k.cin, go, k.cout, d_g + k.w, d, h, w);
+            conv_wgrad_tile_kernel<64><<<grid, 256, 0, st>>>(in.a, k.cin, go, k.cout, d_g + k.w, d, h, w);
         } else if (k.cout > 16) {
-            conv_wgrad_tile_kernel<32><<<dim3(gx, nci, 1), 256, 0, st>>>(in, k.cin, go, k.cout, d_g + k.w, d, h, w);
+            conv_wgrad_tile_kernel<32><<<dim3(gx, nci, 1), 256, 0, st>>>(in.a, k.cin, go, k.cout, d_g + k.w, d, h, w);
         } else {
-            conv_wgrad_tile_kernel<16><<<dim3(gx, nci, 1), 256, 0, st>>>(in, k.cin, go, k.cout, d_g + k.w, d, h, w);
+            conv_wgrad_tile_kernel<16><<<dim3(gx, nci, 1), 256, 0, st>>>(in.a, k.cin, go, k.cout, d_g + k.w, d, h, w);
         }
         const int lanes = std::max(1, 256 / k.cout);
         bias_grad_kernel<<<grid_for(V, lanes), lanes * k.cout, 0, st>>>(go, V, k.cout, d_g + k.b);
     }
-    if (gin) {
-        tile_weights_kernel<<<grid_for(27LL * k.cin * k.cout), 256, 0, st>>>(d_pb + k.w, k.cin, k.cout, 1, d_wt);
-        conv_tiles(go, k.cout, nullptr, gin, k.cin, l, false);
-    }
+    if (gin) conv_tiles(i, true, plain(go, k.cout), k.cout, nullptr, gin, k.cin, l, false);
+}
+
+// the upsampled output of the next coarser decoder level, coarse (C[l + 1] channels)
+ConvIn UNet::decoder_in(int i, int l, const bf16 *coarse) const
+{
+    const int n = convs[i].cin;
+    return in_place(i, l) ? ConvIn{coarse, nullptr, n, 0, 1} : plain(up[l], n);
+}
+
+// [u, skip] of decoder level l
+ConvIn UNet::skip_in(int i, int l) const
+{
+    const int n = convs[i].cin;
+    return in_place(i, l) ? ConvIn{u[l], act[l][1], n / 2, n / 2, 0} : plain(cat[l], n);
 }
 
 int UNet::forward(const float *d_in)
@@ -1257,8 +1293,9 @@ int UNet::forward(const float *d_in)
     int ci = 0;
     const bf16 *x = x0;
     for (int l = 0; l < 4; l++) {
-        conv(ci++, x, act[l][0], l, true);
-        conv(ci++, act[l][0], act[l][1], l, true);
+        conv(ci, plain(x, convs[ci].cin), act[l][0], l, true);
+        conv(ci + 1, plain(act[l][0], C[l]), act[l][1], l, true);
+        ci += 2;
         if (l < 3) {
             if (C[l] % 8 == 0)
                 maxpool8_kernel<<<grid_for(vox(l + 1) * C[l] / 8), 256, 0, st>>>(
@@ -1272,20 +1309,24 @@ int UNet::forward(const float *d_in)
     }
     const bf16 *y = act[3][1];
     for (int l = 2; l >= 0; l--) {
-        if (C[l + 1] % 8 == 0)
+        if (in_place(ci, l)) {
+        } else if (C[l + 1] % 8 == 0)
             upsample8_kernel<<<grid_for(vox(l) * C[l + 1] / 8), 256, 0, st>>>(y, C[l + 1], D >> (l + 1),
                                                                              H >> (l + 1), W >> (l + 1), up[l]);
         else
             upsample_kernel<<<grid_for(vox(l) * C[l + 1]), 256, 0, st>>>(y, C[l + 1], D >> (l + 1), H >> (l + 1),
                                                                          W >> (l + 1), up[l]);
-        conv(ci++, up[l], u[l], l, true);
-        if (C[l] % 8 == 0)
+        conv(ci, decoder_in(ci, l, y), u[l], l, true);
+        ci++;
+        if (in_place(ci, l)) {
+        } else if (C[l] % 8 == 0)
             concat8_kernel<<<grid_for(vox(l) * 2 * C[l] / 8), 256, 0, st>>>(u[l], C[l], act[l][1], C[l], vox(l),
                                                                            cat[l]);
         else
             concat_kernel<<<grid_for(vox(l) * 2 * C[l]), 256, 0, st>>>(u[l], C[l], act[l][1], C[l], vox(l), cat[l]);
-        conv(ci++, cat[l], dec[l][0], l, true);
-        conv(ci++, dec[l][0], dec[l][1], l, true);
+        conv(ci, skip_in(ci, l), dec[l][0], l, true);
+        conv(ci + 1, plain(dec[l][0], C[l]), dec[l][1], l, true);
+        ci += 2;
         y = dec[l][1];
     }
     head_kernel<<<grid_for(vox(0)), 256, 0, st>>>(y, c, d_p + head_w, d_p + head_b, d_in, vox(0), 1.0f / scale, out);
@@ -1312,8 +1353,8 @@ int UNet::backward(const float *d_target, double *loss)
     // decoder, finest level first
     for (int l = 0; l <= 2; l++) {
         const int i2 = ci--, i1 = ci--, iu = ci--;
-        conv_back(i2, dec[l][0], dec[l][1], gdec[l][1], gdec[l][0], l);
-        conv_back(i1, cat[l], dec[l][0], gdec[l][0], gcat[l], l);
+        conv_back(i2, plain(dec[l][0], C[l]), dec[l][1], gdec[l][1], gdec[l][0], l);
+        conv_back(i1, skip_in(i1, l), dec[l][0], gdec[l][0], gcat[l], l);
         // split: the upsampled branch's gradient; the skip's gradient starts here
         const bool p8 = C[l] % 8 == 0;
         if (p8)
@@ -1323,7 +1364,7 @@ int UNet::backward(const float *d_target, double *loss)
         else
             split_grad_kernel<<<grid_for(vox(l) * 2 * C[l]), 256, 0, st>>>(gcat[l], C[l], C[l], vox(l), gu[l],
                                                                            gact[l][1]);
-        conv_back(iu, up[l], u[l], gu[l], gup[l], l);
+        conv_back(iu, decoder_in(iu, l, l == 2 ? act[3][1] : dec[l + 1][1]), u[l], gu[l], gup[l], l);
         bf16 *gy = (l == 2) ? gact[3][1] : gdec[l + 1][1];
         if (C[l + 1] % 8 == 0)
             upsample_grad8_kernel<<<grid_for(vox(l + 1) * C[l + 1] / 8), 256, 0, st>>>(
@@ -1344,9 +1385,9 @@ int UNet::backward(const float *d_target, double *loss)
         else if (l < 3)
             maxpool_grad_kernel<<<grid_for(vox(l + 1) * C[l]), 256, 0, st>>>(act[l][1], pool[l], gpool[l], C[l],
                                                                              D >> l, H >> l, W >> l, gact[l][1], 1);
-        conv_back(ib, act[l][0], act[l][1], gact[l][1], gact[l][0], l);
+        conv_back(ib, plain(act[l][0], C[l]), act[l][1], gact[l][1], gact[l][0], l);
         bf16 *gx = l > 0 ? gpool[l - 1] : nullptr;
-        conv_back(ia, l > 0 ? pool[l - 1] : x0, act[l][0], gact[l][0], gx, l);
+        conv_back(ia, plain(l > 0 ? pool[l - 1] : x0, convs[ia].cin), act[l][0], gact[l][0], gx, l);
     }
     e = cudaGetLastError();
     if (conv_err) {
@@ -1367,6 +1408,7 @@ int UNet::step(float lr)
     const float c1 = 1.0f - std::pow(b1, (float)steps), c2 = 1.0f - std::pow(b2, (float)steps);
     adam_kernel<<<grid_for((long long)n_params), 256, 0, st>>>(d_p, d_g, d_m, d_v, (long long)n_params, lr, b1, b2,
                                                                1e-8f, c1, c2, d_pb);
+    weights_changed();
     cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 0 : fail("U-Net update failed: %s", cudaGetErrorString(e));
 }
@@ -1468,6 +1510,7 @@ int mbirgpu_unet_set_params(mbirgpu_unet *up, const float *params)
     if (e != cudaSuccess) return fail("copy failed: %s", cudaGetErrorString(e));
     mbirgpu::copy_to_bf16_kernel<<<mbirgpu::grid_for((long long)u->n_params), 256, 0, u->st>>>(
         u->d_p, (long long)u->n_params, u->d_pb);
+    u->weights_changed();
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(u->st);
     return e == cudaSuccess ? 0 : fail("U-Net parameter upload failed: %s", cudaGetErrorString(e));

@@ -56,6 +56,7 @@
 #include <cstdint>
 #include <cstdio>
 
+#include "conv_tc.h"
 #include "mbir_internal.h"
 
 namespace mbirgpu {
@@ -209,7 +210,7 @@ __device__ __forceinline__ void tile_coords(const Grid &g, int t, int &x0, int &
 
 template <int NT>
 __global__ void __launch_bounds__(kThreads, 1)
-    conv_tc_kernel(const bf16 *__restrict__ in, int Kin, const bf16 *__restrict__ wtc,
+    conv_tc_kernel(const ConvIn in, const bf16 *__restrict__ wtc,
                    const float *__restrict__ bias, bf16 *__restrict__ out, int Nout, Grid g, int relu)
 {
     using C = Cfg<NT>;
@@ -288,8 +289,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                                   hx = rr - hy * HX;
                         const int z = z0 + hz - 1, y = y0 + hy - 1, x = x0 + hx - 1;
                         const bool inb = z >= zf0 && z < zf1 && z < g.d && y >= 0 && y < g.h && x >= 0 && x < g.w;
-                        const bf16 *src =
-                            inb ? in + (((long long)z * g.h + y) * g.w + x) * Kin + c * 16 + (e & 1) * 8 : in;
+                        const bf16 *src = inb ? in.piece(z, y, x, g.h, g.w, c * 16 + (e & 1) * 8) : in.a;
                         const uint32_t dst = st + (uint32_t)((e & 1) * kHalfBytes + (e >> 1) * 16);
                         asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src),
                                      "r"(inb ? 16 : 0)
@@ -407,12 +407,23 @@ __global__ void __launch_bounds__(kThreads, 1)
 // wtc[ns][c][tap][g][half][r][k] = wt[tap][ns NT + 8 g + r][16 c + 8 half + k]:
 // each (ns, chunk) block is the shared-memory image of the chunk's B operands
 // (27 taps of NT x 16, K-major core matrices: 8 rows x 16 bytes, the two
-// 8-channel halves 128 bytes apart, row groups 256 bytes apart).
-__global__ void tc_weights_kernel(const bf16 *__restrict__ wt, int Kin, int Nout, int NT, bf16 *__restrict__ wtc)
+// 8-channel halves 128 bytes apart, row groups 256 bytes apart), with wt[tap][n][k]
+// the forward weights w[tap][k][n] or, for the data gradient, w[26 - tap][n][k].
+// Every convolution of a network in one launch (blockIdx.y: the convolution,
+// blockIdx.z: forward or data gradient), run when the weights change: two launches
+// per convolution and call were 65 of a training step's 140.
+__global__ void tc_weights_kernel(const ConvTcWeights *__restrict__ list, const bf16 *__restrict__ params,
+                                  bf16 *__restrict__ out)
 {
-    const long long n = 27LL * Nout * Kin;
-    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-        long long r = i;
+    const ConvTcWeights c_ = list[blockIdx.y];
+    const int flip = blockIdx.z, Kin = flip ? c_.cout : c_.cin, Nout = flip ? c_.cin : c_.cout;
+    const int NT = flip ? c_.nt_grad : c_.nt;
+    if (!NT) return;
+    const bf16 *w = params + c_.w;
+    bf16 *wtc = out + (flip ? c_.out_grad : c_.out);
+    const int n = 27 * Nout * Kin;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        int r = i;
         const int k = (int)(r % 8); r /= 8;
         const int row = (int)(r % 8); r /= 8;
         const int half = (int)(r % 2); r /= 2;
@@ -421,7 +432,7 @@ __global__ void tc_weights_kernel(const bf16 *__restrict__ wt, int Kin, int Nout
         const int c = (int)(r % (Kin / 16));
         const int ns = (int)(r / (Kin / 16));
         const int co = ns * NT + grp * 8 + row, ci = c * 16 + half * 8 + k;
-        wtc[i] = wt[((size_t)tap * Nout + co) * Kin + ci];
+        wtc[i] = flip ? w[((size_t)(26 - tap) * Nout + co) * Kin + ci] : w[((size_t)tap * Kin + ci) * Nout + co];
     }
 }
 
@@ -438,7 +449,7 @@ int sm_count()
 }
 
 template <int NT>
-int launch(const bf16 *in, int Kin, const bf16 *wtc, const float *bias, bf16 *out, int Nout, const Grid &g, int relu,
+int launch(const ConvIn &in, const bf16 *wtc, const float *bias, bf16 *out, int Nout, const Grid &g, int relu,
            cudaStream_t st)
 {
     static bool attr = false;
@@ -450,8 +461,8 @@ int launch(const bf16 *in, int Kin, const bf16 *wtc, const float *bias, bf16 *ou
     }
     // CTAs per N slice: one per SM in all, at most one per tile
     const int per_slice = std::max(1, std::min(g.tiles, sm_count() / g.nsplit));
-    conv_tc_kernel<NT><<<(unsigned)(per_slice * g.nsplit), kThreads, Cfg<NT>::kSmem, st>>>(in, Kin, wtc, bias, out,
-                                                                                          Nout, g, relu);
+    conv_tc_kernel<NT><<<(unsigned)(per_slice * g.nsplit), kThreads, Cfg<NT>::kSmem, st>>>(in, wtc, bias, out, Nout, g,
+                                                                                          relu);
     const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? 1 : fail("tensor-core convolution launch failed: %s", cudaGetErrorString(e));
 }
@@ -466,16 +477,27 @@ int conv_tc_split(int Kin, int Nout)
     return Nout % 64 == 0 ? 64 : Nout % 32 == 0 ? 32 : 16;
 }
 
+bool conv_tc_serves(int Kin, int Nout, int d, int df)
+{
+    return conv_tc_split(Kin, Nout) && !(d != df && df % TZ) && d % df == 0;
+}
+
+// The re-laid weights of n convolutions (device list) from the network's
+// parameters, 27 cin cout bf16 at each out / out_grad.
+void conv_tc_weights(const ConvTcWeights *list, int n, const __nv_bfloat16 *params, __nv_bfloat16 *out, cudaStream_t st)
+{
+    tc_weights_kernel<<<dim3(64, n, 2), 256, 0, st>>>(list, params, out);
+}
+
 // out = act(conv(in)) on a grid of d slices (a stack of d / df frames of df
-// slices, zero padding per frame) with weights wt in [27][Nout][Kin]; wtc is
-// scratch of 27 Nout Kin bf16 for the re-laid weights. Returns 1 when
-// launched, 0 when the shape is not served (the caller runs its other
-// kernel), -1 on an error.
-int conv_tc_launch(const __nv_bfloat16 *in, int Kin, const __nv_bfloat16 *wt, __nv_bfloat16 *wtc, const float *bias,
-                   __nv_bfloat16 *out, int Nout, int d, int h, int w, int df, int relu, cudaStream_t st)
+// slices, zero padding per frame) with weights re-laid by conv_tc_weights.
+// Returns 1 when launched, 0 when the shape is not served (the caller runs its
+// other kernel), -1 on an error.
+int conv_tc_launch(const ConvIn &in, int Kin, const __nv_bfloat16 *wtc, const float *bias, __nv_bfloat16 *out,
+                   int Nout, int d, int h, int w, int df, int relu, cudaStream_t st)
 {
     const int NT = conv_tc_split(Kin, Nout);
-    if (!NT || (d != df && df % TZ) || d % df) return 0;
+    if (!conv_tc_serves(Kin, Nout, d, df)) return 0;
     Grid g;
     g.d = d;
     g.h = h;
@@ -488,13 +510,10 @@ int conv_tc_launch(const __nv_bfloat16 *in, int Kin, const __nv_bfloat16 *wt, __
     g.tiles = (int)tiles;
     g.nsplit = Nout / NT;
     g.nchunks = Kin / 16;
-    tc_weights_kernel<<<(unsigned)std::min<long long>((27LL * Nout * Kin + 255) / 256, 4096), 256, 0, st>>>(wt, Kin,
-                                                                                                           Nout, NT,
-                                                                                                           wtc);
     switch (NT) {
-    case 64: return launch<64>(in, Kin, wtc, bias, out, Nout, g, relu, st);
-    case 32: return launch<32>(in, Kin, wtc, bias, out, Nout, g, relu, st);
-    default: return launch<16>(in, Kin, wtc, bias, out, Nout, g, relu, st);
+    case 64: return launch<64>(in, wtc, bias, out, Nout, g, relu, st);
+    case 32: return launch<32>(in, wtc, bias, out, Nout, g, relu, st);
+    default: return launch<16>(in, wtc, bias, out, Nout, g, relu, st);
     }
 }
 
