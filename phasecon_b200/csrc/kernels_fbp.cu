@@ -71,13 +71,13 @@ void launch_mask_object(const Geom &g, const uint8_t *d_mask, float *d_x, cudaSt
     mask_object_kernel<<<148 * 8, 256, 0, st>>>(g.N_time, g.N_x * g.N_y, g.N_z, d_mask, d_x);
 }
 
-void launch_fbp(const Geom &g, const uint32_t *d_table, const int32_t *d_view_first, const int32_t *d_views,
+void launch_fbp(const Geom &g, const uint32_t *d_table, const int32_t *d_view_first,
                 const float *d_y, float *d_q, float *d_x, cudaStream_t st)
 {
     const size_t smem = ((size_t)g.N_r * g.N_t + 2 * (size_t)g.N_r) * sizeof(float);
     cudaFuncSetAttribute(ramp_filter_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     ramp_filter_kernel<<<g.N_p, 256, smem, st>>>(g.N_r, g.N_t, g.delta_r, d_y, d_q);
-    launch_back_project(g, d_table, d_view_first, d_views, d_q, d_x, st);
+    launch_back_project(g, d_table, d_view_first, d_q, d_x, st);
     const size_t per_frame = (size_t)g.N_x * g.N_y * g.N_z;
     fbp_scale_kernel<<<148 * 8, 256, 0, st>>>(g.N_time, per_frame, d_view_first, d_x);
 }

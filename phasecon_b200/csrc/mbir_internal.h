@@ -97,12 +97,12 @@ size_t variance_scratch_doubles();
 int variance_update(const Geom &g, int N_p, const float *d_err, float *d_w, double *var_est, double *d_scratch,
                     cudaStream_t st);
 void launch_back_project(const Geom &g, const uint32_t *d_table, const int32_t *d_view_first,
-                         const int32_t *d_views, const float *d_sino, float *d_x, cudaStream_t st);
+                         const float *d_sino, float *d_x, cudaStream_t st);
 
 // Filtered back-projection of d_y into d_x ([N_time][N_y][N_x][N_z]); d_q is a
 // sinogram-sized scratch for the ramp-filtered data. The ramp filter keeps one
 // view ([N_r][N_t] floats) in shared memory.
-void launch_fbp(const Geom &g, const uint32_t *d_table, const int32_t *d_view_first, const int32_t *d_views,
+void launch_fbp(const Geom &g, const uint32_t *d_table, const int32_t *d_view_first,
                 const float *d_y, float *d_q, float *d_x, cudaStream_t st);
 // Zero the voxel columns of d_x ([N_time][N_y][N_x][N_z]) outside the
 // reconstruction circle: ICD never updates them, and the reference keeps them 0.

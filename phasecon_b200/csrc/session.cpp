@@ -650,7 +650,7 @@ int Session::back_project(const float *sino, float *obj)
         return -1;
     }
     cudaError_t e = cudaMemcpyAsync(d_s, sino, n_sino * sizeof(float), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) launch_back_project(g, d_table, d_view_first, d_views, d_s, d_o, st);
+    if (e == cudaSuccess) launch_back_project(g, d_table, d_view_first, d_s, d_o, st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e == cudaSuccess) {
         launch_zfast_to_vol(d_o, d_tmp, g.N_time, g.N_z, g.N_y, g.N_x, st);
@@ -670,7 +670,7 @@ int Session::fbp(float *obj)
     float *d_o = nullptr;
     size_t acc = 0;
     if (dalloc(&d_o, n_vox, &acc)) return -1;
-    launch_fbp(g, d_table, d_view_first, d_views, d_y, d_tmp, d_o, st);
+    launch_fbp(g, d_table, d_view_first, d_y, d_tmp, d_o, st);
     launch_zfast_to_vol(d_o, d_tmp, g.N_time, g.N_z, g.N_y, g.N_x, st);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(obj, d_tmp, n_vox * sizeof(float), cudaMemcpyDeviceToHost, st);
@@ -684,7 +684,7 @@ int Session::set_object_fbp()
 {
     const Geom &g = hs.g;
     if (!fbp_supported(g)) return fail("FBP: %d channels x %d rows per view exceed the filter's shared memory", g.N_r, g.N_t);
-    launch_fbp(g, d_table, d_view_first, d_views, d_y, d_tmp, d_x, st);
+    launch_fbp(g, d_table, d_view_first, d_y, d_tmp, d_x, st);
     launch_mask_object(g, d_mask, d_x, st);
     CK(cudaGetLastError());
     return refresh_error();
@@ -740,7 +740,7 @@ int Session::set_object_unet(UNet *u)
     if (!fbp_supported(g)) return fail("FBP: %d channels x %d rows per view exceed the filter's shared memory", g.N_r, g.N_t);
     // d_tmp (max(sinogram, volume) floats) holds the filtered sinogram during
     // the FBP, then the volume in the network's [T][Z][Y][X] layout
-    launch_fbp(g, d_table, d_view_first, d_views, d_y, d_tmp, d_x, st);
+    launch_fbp(g, d_table, d_view_first, d_y, d_tmp, d_x, st);
     launch_zfast_to_vol(d_x, d_tmp, g.N_time, g.N_z, g.N_y, g.N_x, st);
     cudaError_t e = cudaStreamSynchronize(st);  // the network runs on its own stream
     int rc = e == cudaSuccess ? unet_apply_frames(u, d_tmp, g.N_time, g.N_z, g.N_y, g.N_x) : -1;
