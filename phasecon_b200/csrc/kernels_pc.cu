@@ -10,9 +10,9 @@
 // so every pass reads and writes the view once. FFTs are Stockham autosort
 // stages of radix up to 16 (the R points of a butterfly in registers,
 // ping-pong between two shared-memory buffers; for 256-point sequences the
-// points stay in registers with one shared-memory exchange per transform)
-// with twiddles exp(-2 pi i m / n_max) precomputed in double and rounded once
-// to float.
+// points stay in registers with one shared-memory exchange per transform).
+// Factors inside a butterfly are constants; those between stages,
+// exp(-2 pi i m / n_max), are computed in double and rounded once to float.
 // Per-view sums needed by the steepest-descent step size and the stopping
 // tests are block-reduced and added in FP64. Views whose loop has stopped
 // (per-view flags) skip every launch.
@@ -39,10 +39,11 @@ __device__ __forceinline__ int fpos(int q, int i, int sstride) { return q * sstr
 
 // exp(-+ 2 pi i m / nmax), 0 <= m < nmax, from the full-circle table the
 // kernels keep in shared memory (load_twiddles).
-__device__ __forceinline__ float2 twid(const float2 *tw, int m, int nmax, bool inverse)
+template <bool INV>
+__device__ __forceinline__ float2 twid(const float2 *tw, int m)
 {
     float2 w = tw[m];
-    if (inverse) w.y = -w.y;
+    if (INV) w.y = -w.y;
     return w;
 }
 
@@ -56,26 +57,53 @@ __host__ __device__ constexpr int bit_reverse(int i, int bits)
 
 __host__ __device__ constexpr int log2_const(int n) { return n <= 1 ? 0 : 1 + log2_const(n >> 1); }
 
+// a + w t and a - w t for w = exp(-2 pi i k / len) (its conjugate for an inverse
+// transform), k and len constants up to 16: additions where w is 1 or -i, else two
+// fused steps a component
+template <bool INV>
+__device__ __forceinline__ void butterfly(float2 &a, float2 &t, int k16)
+{
+    constexpr float c1 = 0.923879532511286756f, s1 = 0.382683432365089772f, h = 0.707106781186547524f;
+    // exp(-2 pi i k16 / 16); k16 is a constant once the loops are unrolled
+    const int m = k16 < 4 ? k16 : 8 - k16;  // 1, 2 or 3 where it is used
+    const float cx = m == 1 ? c1 : m == 2 ? h : s1, sy = m == 1 ? s1 : m == 2 ? h : c1;
+    const float x = k16 < 4 ? cx : -cx, y = INV ? sy : -sy;
+    const float2 u = a;
+    if (k16 == 0) {
+        a = cadd(u, t);
+        t = csub(u, t);
+    } else if (k16 == 4) {
+        const float2 r = INV ? make_float2(-t.y, t.x) : make_float2(t.y, -t.x);
+        a = cadd(u, r);
+        t = csub(u, r);
+    } else {
+        a = make_float2(fmaf(x, t.x, fmaf(-y, t.y, u.x)), fmaf(x, t.y, fmaf(y, t.x, u.y)));
+        t = make_float2(fmaf(-x, t.x, fmaf(y, t.y, u.x)), fmaf(-x, t.y, fmaf(-y, t.x, u.y)));
+    }
+}
+
+// the stages of sub-transforms of len points and up
+template <int R, bool INV, int len>
+__device__ __forceinline__ void dft_stage(float2 (&y)[R])
+{
+#pragma unroll
+    for (int b = 0; b < R / 2; b++) {
+        const int k = b % (len / 2), i = b / (len / 2) * len + k;
+        butterfly<INV>(y[i], y[i + len / 2], k * (16 / len));
+    }
+    if constexpr (len < R) dft_stage<R, INV, 2 * len>(y);
+}
+
 // R-point DFT of x in registers, natural order in and out (radix-2
-// decimation in time over a bit-reversed copy; every index is a constant).
-template <int R>
-__device__ __forceinline__ void dft_regs(float2 (&x)[R], const float2 *tw, int nmax, bool inverse)
+// decimation in time over a bit-reversed copy; every index and factor is a constant).
+template <int R, bool INV>
+__device__ __forceinline__ void dft_regs(float2 (&x)[R])
 {
     constexpr int bits = log2_const(R);
     float2 y[R];
 #pragma unroll
     for (int i = 0; i < R; i++) y[bit_reverse(i, bits)] = x[i];
-#pragma unroll
-    for (int len = 2; len <= R; len <<= 1) {
-#pragma unroll
-        for (int i = 0; i < R; i += len)
-#pragma unroll
-            for (int k = 0; k < len / 2; k++) {
-                const float2 t = cmul(twid(tw, k * (nmax / len), nmax, inverse), y[i + k + len / 2]);
-                y[i + k + len / 2] = csub(y[i + k], t);
-                y[i + k] = cadd(y[i + k], t);
-            }
-    }
+    dft_stage<R, INV, 2>(y);
 #pragma unroll
     for (int i = 0; i < R; i++) x[i] = y[i];
 }
@@ -85,9 +113,9 @@ __device__ __forceinline__ void dft_regs(float2 (&x)[R], const float2 *tw, int n
 // takes x_p = a[j + p n / R], p < R, multiplies x_p by w_{RL}^{p (j mod L)},
 // transforms the R points in registers and writes them to b at
 // (j - j mod L) R + j mod L + p L.
-template <int R>
+template <int R, bool INV>
 __device__ __forceinline__ void stockham_stage(const float2 *a, float2 *b, int n, int log2n, int L, int nseq,
-                                               int sstride, const float2 *tw, int nmax, bool inverse)
+                                               int sstride, const float2 *tw, int nmax)
 {
     constexpr int lr = log2_const(R);
     const int lm = log2n - lr;  // butterflies per sequence: n / R = 2^lm
@@ -101,9 +129,9 @@ __device__ __forceinline__ void stockham_stage(const float2 *a, float2 *b, int n
         for (int p = 0; p < R; p++) x[p] = a[fpos(q, j + p * m, sstride)];
         if (L > 1) {
 #pragma unroll
-            for (int p = 1; p < R; p++) x[p] = cmul(twid(tw, k * p * tscale, nmax, inverse), x[p]);
+            for (int p = 1; p < R; p++) x[p] = cmul(twid<INV>(tw, k * p * tscale), x[p]);
         }
-        dft_regs<R>(x, tw, nmax, inverse);
+        dft_regs<R, INV>(x);
         const int o = ((j - k) << lr) + k;
 #pragma unroll
         for (int p = 0; p < R; p++) b[fpos(q, o + p * L, sstride)] = x[p];
@@ -114,22 +142,23 @@ __device__ __forceinline__ void stockham_stage(const float2 *a, float2 *b, int n
 // stages of radix max_radix (16, 8, 4 or 2; smaller for the rest) ping-pong
 // between a and b.
 // Returns the buffer holding the result.
+template <bool INV>
 __device__ float2 *fft_smem(float2 *a, float2 *b, int n, int log2n, int nseq, int sstride, const float2 *tw,
-                            int nmax, bool inverse, int max_radix)
+                            int nmax, int max_radix)
 {
     for (int L = 1; L < n;) {
         const int rem = n / L < max_radix ? n / L : max_radix;
         if (rem >= 16) {
-            stockham_stage<16>(a, b, n, log2n, L, nseq, sstride, tw, nmax, inverse);
+            stockham_stage<16, INV>(a, b, n, log2n, L, nseq, sstride, tw, nmax);
             L <<= 4;
         } else if (rem >= 8) {
-            stockham_stage<8>(a, b, n, log2n, L, nseq, sstride, tw, nmax, inverse);
+            stockham_stage<8, INV>(a, b, n, log2n, L, nseq, sstride, tw, nmax);
             L <<= 3;
         } else if (rem >= 4) {
-            stockham_stage<4>(a, b, n, log2n, L, nseq, sstride, tw, nmax, inverse);
+            stockham_stage<4, INV>(a, b, n, log2n, L, nseq, sstride, tw, nmax);
             L <<= 2;
         } else {
-            stockham_stage<2>(a, b, n, log2n, L, nseq, sstride, tw, nmax, inverse);
+            stockham_stage<2, INV>(a, b, n, log2n, L, nseq, sstride, tw, nmax);
             L <<= 1;
         }
         __syncthreads();
@@ -195,8 +224,10 @@ __device__ __forceinline__ float2 expz_fast(float zr, float zi)
 constexpr int kStage = 8;
 
 namespace {
-// prologue input of element i (pixel p of the view)
-__device__ __forceinline__ float2 prologue_in(const PcArgs &A, int prologue, size_t i, size_t p)
+// prologue input of element i (pixel p of the view). The operation is a template
+// parameter: a switch per element kept a pass's loads from overlapping.
+template <int prologue>
+__device__ __forceinline__ float2 prologue_in(const PcArgs &A, size_t i, size_t p)
 {
     switch (prologue) {
     case PC_IN_DW: return cscale(__ldg(A.in + i), __ldg(A.D + p));
@@ -215,7 +246,8 @@ struct EpiIn {
     float s0, s1;
 };
 
-__device__ __forceinline__ EpiIn epilogue_in(const PcArgs &A, int epilogue, size_t i, size_t p)
+template <int epilogue>
+__device__ __forceinline__ EpiIn epilogue_in(const PcArgs &A, size_t i, size_t p)
 {
     EpiIn r = {make_float2(0.f, 0.f), make_float2(0.f, 0.f), 1.f, 0.f};
     switch (epilogue) {
@@ -248,8 +280,8 @@ __device__ __forceinline__ EpiIn epilogue_in(const PcArgs &A, int epilogue, size
 }
 
 // writes element i's epilogue result; returns its term of the per-view sum
-__device__ __forceinline__ double epilogue_out(const PcDims &d, const PcArgs &A, int epilogue, size_t i, float2 t,
-                                               const EpiIn &in)
+template <int epilogue>
+__device__ __forceinline__ double epilogue_out(const PcDims &d, const PcArgs &A, size_t i, float2 t, const EpiIn &in)
 {
     switch (epilogue) {
     case PC_OUT_GRES: {  // conj(Omega) Lambda (Omega t - y)
@@ -294,7 +326,8 @@ __device__ __forceinline__ int ilog2_pow2(int n) { return 31 - __clz(n); }
 }  // namespace
 
 // ---------------------------------------------------------------------------- pass 1
-__global__ void pc_rows_forward(PcDims d, PcArgs A, int prologue)
+template <int prologue>
+__global__ void pc_rows_forward(PcDims d, PcArgs A)
 {
     extern __shared__ float2 smem[];
     const int v = blockIdx.y;
@@ -311,7 +344,7 @@ __global__ void pc_rows_forward(PcDims d, PcArgs A, int prologue)
 #pragma unroll
         for (int u = 0; u < kStage; u++) {
             const int e = e0 + u * blockDim.x;
-            if (e < total) x[u] = prologue_in(A, prologue, vb + pb + e, pb + e);
+            if (e < total) x[u] = prologue_in<prologue>(A, vb + pb + e, pb + e);
         }
 #pragma unroll
         for (int u = 0; u < kStage; u++) {
@@ -320,7 +353,7 @@ __global__ void pc_rows_forward(PcDims d, PcArgs A, int prologue)
         }
     }
     __syncthreads();
-    float2 *res = fft_smem(a, b, C, lc, nrows, S, s_tw, d.nmax, false, d.fft_radix);
+    float2 *res = fft_smem<false>(a, b, C, lc, nrows, S, s_tw, d.nmax, d.fft_radix);
     for (int e = threadIdx.x; e < total; e += blockDim.x) A.work[vb + pb + e] = res[fpos(e >> lc, e & (C - 1), S)];
 }
 
@@ -350,7 +383,7 @@ __global__ void pc_cols_filter(PcDims d, PcArgs A, const float2 *__restrict__ tr
         }
     }
     __syncthreads();
-    float2 *res = fft_smem(a, b, R, d.logR, cb, S, s_tw, d.nmax, false, d.fft_radix);
+    float2 *res = fft_smem<false>(a, b, R, d.logR, cb, S, s_tw, d.nmax, d.fft_radix);
     float2 *other = res == a ? b : a;
     for (int e0 = threadIdx.x; e0 < total; e0 += kStage * blockDim.x) {
         float2 h[kStage];
@@ -369,13 +402,14 @@ __global__ void pc_cols_filter(PcDims d, PcArgs A, const float2 *__restrict__ tr
         }
     }
     __syncthreads();
-    res = fft_smem(res, other, R, d.logR, cb, S, s_tw, d.nmax, true, d.fft_radix);
+    res = fft_smem<true>(res, other, R, d.logR, cb, S, s_tw, d.nmax, d.fft_radix);
     for (int e = threadIdx.x; e < total; e += blockDim.x)
         A.work[vb + (size_t)(e >> lcb) * C + c0 + (e & (cb - 1))] = res[fpos(e & (cb - 1), e >> lcb, S)];
 }
 
 // ---------------------------------------------------------------------------- pass 3
-__global__ void pc_rows_inverse(PcDims d, PcArgs A, int epilogue)
+template <int epilogue>
+__global__ void pc_rows_inverse(PcDims d, PcArgs A)
 {
     extern __shared__ float2 smem[];
     __shared__ double s_red[32];
@@ -402,7 +436,7 @@ __global__ void pc_rows_inverse(PcDims d, PcArgs A, int epilogue)
         }
     }
     __syncthreads();
-    float2 *res = fft_smem(a, b, C, lc, nrows, S, s_tw, d.nmax, true, d.fft_radix);
+    float2 *res = fft_smem<true>(a, b, C, lc, nrows, S, s_tw, d.nmax, d.fft_radix);
     const float inv_n = 1.0f / (float)d.N;
     double acc = 0.0;
     constexpr int kEpi = kStage / 2;  // the epilogues read up to two complex operands per element
@@ -411,13 +445,13 @@ __global__ void pc_rows_inverse(PcDims d, PcArgs A, int epilogue)
 #pragma unroll
         for (int u = 0; u < kEpi; u++) {
             const int e = e0 + u * blockDim.x;
-            if (e < total) in[u] = epilogue_in(A, epilogue, vb + pb + e, pb + e);
+            if (e < total) in[u] = epilogue_in<epilogue>(A, vb + pb + e, pb + e);
         }
 #pragma unroll
         for (int u = 0; u < kEpi; u++) {
             const int e = e0 + u * blockDim.x;
             if (e < total)
-                acc += epilogue_out(d, A, epilogue, vb + pb + e, cscale(res[fpos(e >> lc, e & (C - 1), S)], inv_n),
+                acc += epilogue_out<epilogue>(d, A, vb + pb + e, cscale(res[fpos(e >> lc, e & (C - 1), S)], inv_n),
                                     in[u]);
         }
     }
@@ -435,43 +469,60 @@ __global__ void pc_rows_inverse(PcDims d, PcArgs A, int epilogue)
 // the generic passes' two radix-16 stages; one shared-memory exchange per
 // transform instead of four, and one barrier instead of four. A CTA holds 16
 // sequences (256 threads).
+// What bounds them: the latency of a CTA's load, transform and store phases (94 MB
+// in and out would take 29 us). 180 views of 256 x 256, rows forward / columns /
+// rows inverse with its epilogue: 31 / 53 / 43 to 64 us; with the factors inside a
+// butterfly read from the shared table, that table's bank conflicts and a switch
+// per element for the prologue and epilogue 45 to 81 / 63 / 82 to 106. Four CTAs an SM
+// for the rows (three: the same), two for the columns (three and four 62).
 namespace {
 constexpr int kF = 16;  // sequences per CTA and points per thread
 
-// stage 2 of a 256-point transform on this thread's points x[p] = a[j + 16p]:
-// twiddles w_256^(p j) (twiddle index scaled to the table's nmax), then the
-// 16-point DFT; outputs X[j + 16p] in x[p]
-__device__ __forceinline__ void stage2_256(float2 (&x)[kF], int j, const float2 *tw, int nmax, bool inverse)
+// The twiddles of stage 2, w_256^(p j), at 16 p + j: a warp's 16 butterflies j read
+// neighbouring entries (the full circle indexed by p j had up to eight on a bank).
+__device__ __forceinline__ void load_twiddles_256(float2 *s_tw, const float2 *tw, int nmax)
 {
-    const int sc = nmax >> 8;
+    const int m = ((threadIdx.x >> 4) * (threadIdx.x & 15) & 255) * (nmax >> 8), h = nmax / 2;
+    const float2 w = __ldg(tw + (m < h ? m : m - h));
+    s_tw[threadIdx.x] = m < h ? w : make_float2(-w.x, -w.y);
+}
+
+// a 256-point transform over the sequences' threads: x[p] is point j + 16 p before and
+// after. The caller's barrier (or the one here) stands between the twiddles' stores and
+// their use and, with sync_first, between an earlier transform's reads of a and its reuse.
+template <bool INV>
+__device__ __forceinline__ void fft_256(float2 (&x)[kF], float2 *a, const float2 *s_tw, int q, int j, bool sync_first)
+{
+    const int S = fft_seq_stride(256);
+    dft_regs<kF, INV>(x);  // stage 1 (L = 1): outputs at 16 j + p
+    if (sync_first) __syncthreads();
 #pragma unroll
-    for (int p = 1; p < kF; p++) x[p] = cmul(twid(tw, p * j * sc, nmax, inverse), x[p]);
-    dft_regs<kF>(x, tw, nmax, inverse);
+    for (int p = 0; p < kF; p++) a[fpos(q, 16 * j + p, S)] = x[p];
+    __syncthreads();
+#pragma unroll
+    for (int p = 0; p < kF; p++) {
+        const float2 v = a[fpos(q, j + 16 * p, S)];
+        x[p] = p ? cmul(twid<INV>(s_tw, 16 * p + j), v) : v;
+    }
+    dft_regs<kF, INV>(x);
 }
 }  // namespace
 
-__global__ void __launch_bounds__(256) pc_rows_forward_256(PcDims d, PcArgs A, int prologue)
+template <int prologue>
+__global__ void __launch_bounds__(256, 4) pc_rows_forward_256(PcDims d, PcArgs A)
 {
     extern __shared__ float2 smem[];
     const int v = blockIdx.y;
     if (A.active && !A.active[v]) return;
-    const int S = fft_seq_stride(256);
-    float2 *s_tw = smem, *a = smem + d.nmax;
-    load_twiddles(s_tw, A.tw, d.nmax);
+    float2 *s_tw = smem, *a = smem + 256;
     const int q = threadIdx.x >> 4, j = threadIdx.x & 15;  // sequence (row) of the CTA, butterfly
     const int r = blockIdx.x * kF + q;
     const size_t pb = (size_t)r * 256, vb = (size_t)v * d.N;
     float2 x[kF];
 #pragma unroll
-    for (int p = 0; p < kF; p++) x[p] = prologue_in(A, prologue, vb + pb + j + 16 * p, pb + j + 16 * p);
-    __syncthreads();  // the twiddle table
-    dft_regs<kF>(x, s_tw, d.nmax, false);  // stage 1 (L = 1): outputs at 16 j + p
-#pragma unroll
-    for (int p = 0; p < kF; p++) a[fpos(q, 16 * j + p, S)] = x[p];
-    __syncthreads();
-#pragma unroll
-    for (int p = 0; p < kF; p++) x[p] = a[fpos(q, j + 16 * p, S)];
-    stage2_256(x, j, s_tw, d.nmax, false);
+    for (int p = 0; p < kF; p++) x[p] = prologue_in<prologue>(A, vb + pb + j + 16 * p, pb + j + 16 * p);
+    load_twiddles_256(s_tw, A.tw, d.nmax);
+    fft_256<false>(x, a, s_tw, q, j, false);
 #pragma unroll
     for (int p = 0; p < kF; p++) A.work[vb + pb + j + 16 * p] = x[p];
 }
@@ -481,62 +532,42 @@ __global__ void __launch_bounds__(256, 2) pc_cols_filter_256(PcDims d, PcArgs A,
     extern __shared__ float2 smem[];
     const int v = blockIdx.y;
     if (A.active && !A.active[v]) return;
-    const int C = d.C, S = fft_seq_stride(256);
-    float2 *s_tw = smem, *a = smem + d.nmax;
-    load_twiddles(s_tw, A.tw, d.nmax);
+    const int C = d.C;
+    float2 *s_tw = smem, *a = smem + 256;
     const int q = threadIdx.x & 15, j = threadIdx.x >> 4;  // column of the CTA (fastest: coalesced), butterfly
     const int c = blockIdx.x * kF + q;
-    const size_t vb = (size_t)v * d.N;
+    float2 *z = A.work + (size_t)v * d.N + (size_t)j * C + c;
+    const float2 *h = transfer + (size_t)j * C + c;
     float2 x[kF];
 #pragma unroll
-    for (int p = 0; p < kF; p++) x[p] = A.work[vb + (size_t)(j + 16 * p) * C + c];
-    __syncthreads();  // the twiddle table
-    dft_regs<kF>(x, s_tw, d.nmax, false);
-#pragma unroll
-    for (int p = 0; p < kF; p++) a[fpos(q, 16 * j + p, S)] = x[p];
-    __syncthreads();
-#pragma unroll
-    for (int p = 0; p < kF; p++) x[p] = a[fpos(q, j + 16 * p, S)];
-    stage2_256(x, j, s_tw, d.nmax, false);
+    for (int p = 0; p < kF; p++) x[p] = z[(size_t)16 * p * C];
+    load_twiddles_256(s_tw, A.tw, d.nmax);
+    fft_256<false>(x, a, s_tw, q, j, false);
     // the forward outputs X[j + 16p] are the inverse's stage-1 inputs of the
     // same butterfly j: multiply by the transfer table and go on in registers
 #pragma unroll
-    for (int p = 0; p < kF; p++) x[p] = cmul(x[p], __ldg(transfer + (size_t)(j + 16 * p) * C + c));
-    dft_regs<kF>(x, s_tw, d.nmax, true);
-    __syncthreads();  // every thread has read its stage-2 points
+    for (int p = 0; p < kF; p++) x[p] = cmul(x[p], __ldg(h + (size_t)16 * p * C));
+    fft_256<true>(x, a, s_tw, q, j, true);
 #pragma unroll
-    for (int p = 0; p < kF; p++) a[fpos(q, 16 * j + p, S)] = x[p];
-    __syncthreads();
-#pragma unroll
-    for (int p = 0; p < kF; p++) x[p] = a[fpos(q, j + 16 * p, S)];
-    stage2_256(x, j, s_tw, d.nmax, true);
-#pragma unroll
-    for (int p = 0; p < kF; p++) A.work[vb + (size_t)(j + 16 * p) * C + c] = x[p];
+    for (int p = 0; p < kF; p++) z[(size_t)16 * p * C] = x[p];
 }
 
-__global__ void __launch_bounds__(256, 3) pc_rows_inverse_256(PcDims d, PcArgs A, int epilogue)
+template <int epilogue>
+__global__ void __launch_bounds__(256, 4) pc_rows_inverse_256(PcDims d, PcArgs A)
 {
     extern __shared__ float2 smem[];
     __shared__ double s_red[32];
     const int v = blockIdx.y;
     if (A.active && !A.active[v]) return;
-    const int S = fft_seq_stride(256);
-    float2 *s_tw = smem, *a = smem + d.nmax;
-    load_twiddles(s_tw, A.tw, d.nmax);
+    float2 *s_tw = smem, *a = smem + 256;
     const int q = threadIdx.x >> 4, j = threadIdx.x & 15;
     const int r = blockIdx.x * kF + q;
     const size_t pb = (size_t)r * 256, vb = (size_t)v * d.N;
     float2 x[kF];
 #pragma unroll
     for (int p = 0; p < kF; p++) x[p] = A.work[vb + pb + j + 16 * p];
-    __syncthreads();
-    dft_regs<kF>(x, s_tw, d.nmax, true);
-#pragma unroll
-    for (int p = 0; p < kF; p++) a[fpos(q, 16 * j + p, S)] = x[p];
-    __syncthreads();
-#pragma unroll
-    for (int p = 0; p < kF; p++) x[p] = a[fpos(q, j + 16 * p, S)];
-    stage2_256(x, j, s_tw, d.nmax, true);
+    load_twiddles_256(s_tw, A.tw, d.nmax);
+    fft_256<true>(x, a, s_tw, q, j, false);
     const float inv_n = 1.0f / (float)d.N;
     double acc = 0.0;
     constexpr int kEpi = 4;  // operands of four elements in flight
@@ -546,16 +577,83 @@ __global__ void __launch_bounds__(256, 3) pc_rows_inverse_256(PcDims d, PcArgs A
 #pragma unroll
         for (int u = 0; u < kEpi; u++) {
             const size_t e = pb + j + 16 * (p0 + u);
-            in[u] = epilogue_in(A, epilogue, vb + e, e);
+            in[u] = epilogue_in<epilogue>(A, vb + e, e);
         }
 #pragma unroll
         for (int u = 0; u < kEpi; u++) {
             const size_t e = pb + j + 16 * (p0 + u);
-            acc += epilogue_out(d, A, epilogue, vb + e, cscale(x[p0 + u], inv_n), in[u]);
+            acc += epilogue_out<epilogue>(d, A, vb + e, cscale(x[p0 + u], inv_n), in[u]);
         }
     }
     if (epilogue == PC_OUT_GRAD || epilogue == PC_OUT_SDEN || epilogue == PC_OUT_PCOST)
         block_add(acc, A.acc + (size_t)v * kPcAccSlots + A.acc_slot, s_red);
+}
+
+// ---------------------------------------------------------------------------- launches
+namespace {
+constexpr size_t kSmem256 = (256 + kF * (256 + 256 / 16 + 1)) * sizeof(float2);  // fft_seq_stride(256) = 273
+
+// Allows a generic pass its shared memory, in the call that launches it (allowing every
+// pass when a session starts loads all of them: 37 ms the first time). One limit for all
+// sizes, so that a smaller session's does not lower a larger one's; at most 92 KB are used.
+template <class F>
+void allow_shared(F *pass)
+{
+    cudaFuncSetAttribute(pass, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024);
+}
+
+template <int prologue>
+void rows_forward(const PcDims &d, const PcArgs &A, bool reg256, size_t smem, cudaStream_t st)
+{
+    if (reg256) {
+        pc_rows_forward_256<prologue><<<dim3(d.R / kF, d.V), 256, kSmem256, st>>>(d, A);
+        return;
+    }
+    allow_shared(pc_rows_forward<prologue>);
+    pc_rows_forward<prologue><<<dim3((d.R + d.rows_per_cta - 1) / d.rows_per_cta, d.V), 256, smem, st>>>(d, A);
+}
+
+template <int epilogue>
+void rows_inverse(const PcDims &d, const PcArgs &A, bool reg256, size_t smem, cudaStream_t st)
+{
+    if (reg256) {
+        pc_rows_inverse_256<epilogue><<<dim3(d.R / kF, d.V), 256, kSmem256, st>>>(d, A);
+        return;
+    }
+    allow_shared(pc_rows_inverse<epilogue>);
+    pc_rows_inverse<epilogue><<<dim3((d.R + d.rows_per_cta - 1) / d.rows_per_cta, d.V), 256, smem, st>>>(d, A);
+}
+}  // namespace
+
+void launch_transform(const PcDims &d, const PcArgs &A, size_t smem_rows, size_t smem_cols, int prologue,
+                      const float2 *table, int epilogue, cudaStream_t st)
+{
+    // 256-point sequences with radix-16 stages: the register-resident passes
+    // (16 sequences per CTA; the twiddles and one padded buffer, 37 KB)
+    const bool rows256 = d.C == 256 && d.R % kF == 0 && d.fft_radix == 16;
+    const bool cols256 = d.R == 256 && d.C % kF == 0 && d.fft_radix == 16;
+    switch (prologue) {
+    case PC_IN_DW: rows_forward<PC_IN_DW>(d, A, rows256, smem_rows, st); break;
+    case PC_IN_DEZ: rows_forward<PC_IN_DEZ>(d, A, rows256, smem_rows, st); break;
+    case PC_IN_PAG: rows_forward<PC_IN_PAG>(d, A, rows256, smem_rows, st); break;
+    default: rows_forward<PC_IN_PLAIN>(d, A, rows256, smem_rows, st);
+    }
+    if (cols256) {
+        pc_cols_filter_256<<<dim3(d.C / kF, d.V), 256, kSmem256, st>>>(d, A, table);
+    } else {
+        allow_shared(pc_cols_filter);
+        pc_cols_filter<<<dim3(d.C / d.cols_per_cta, d.V), 256, smem_cols, st>>>(d, A, table);
+    }
+    switch (epilogue) {
+    case PC_OUT_GRES: rows_inverse<PC_OUT_GRES>(d, A, rows256, smem_rows, st); break;
+    case PC_OUT_GRAD: rows_inverse<PC_OUT_GRAD>(d, A, rows256, smem_rows, st); break;
+    case PC_OUT_SFWD: rows_inverse<PC_OUT_SFWD>(d, A, rows256, smem_rows, st); break;
+    case PC_OUT_SDEN: rows_inverse<PC_OUT_SDEN>(d, A, rows256, smem_rows, st); break;
+    case PC_OUT_OMEGA: rows_inverse<PC_OUT_OMEGA>(d, A, rows256, smem_rows, st); break;
+    case PC_OUT_PCOST: rows_inverse<PC_OUT_PCOST>(d, A, rows256, smem_rows, st); break;
+    case PC_OUT_PAG: rows_inverse<PC_OUT_PAG>(d, A, rows256, smem_rows, st); break;
+    default: rows_inverse<PC_OUT_PLAIN>(d, A, rows256, smem_rows, st);
+    }
 }
 
 // ---------------------------------------------------------------------------- pointwise steps

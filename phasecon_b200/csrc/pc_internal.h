@@ -66,14 +66,9 @@ struct PcPrior {
     float f_f[9], T00_f, T01_f, T10_f, T11_f;  // FP32 copies for the per-pixel search
 };
 
-__global__ void pc_rows_forward(PcDims d, PcArgs A, int prologue);
-__global__ void pc_cols_filter(PcDims d, PcArgs A, const float2 *transfer);
-__global__ void pc_rows_inverse(PcDims d, PcArgs A, int epilogue);
-// the same passes for 256-point sequences with radix-16 stages, the points in
-// registers (16 sequences per 256-thread CTA)
-__global__ void pc_rows_forward_256(PcDims d, PcArgs A, int prologue);
-__global__ void pc_cols_filter_256(PcDims d, PcArgs A, const float2 *transfer);
-__global__ void pc_rows_inverse_256(PcDims d, PcArgs A, int epilogue);
+// The three passes of one transform of every view, their form picked by the lengths.
+void launch_transform(const PcDims &d, const PcArgs &A, size_t smem_rows, size_t smem_cols, int prologue,
+                      const float2 *table, int epilogue, cudaStream_t st);
 __global__ void pc_sd_update(PcDims d, PcArgs A);
 __global__ void pc_sd_finish(PcDims d, PcArgs A, int step, float sd_thresh);
 __global__ void pc_pret_prepare(PcDims d, PcArgs A);
