@@ -617,25 +617,34 @@ int Session::amatrix(int32_t *first, int32_t *count, float *values)
     return 0;
 }
 
+// A volume of scratch beside d_tmp: the FP64 accumulator, whose content no call needs
+// from another, where it is large enough (n_vox <= 2 n_sino floats: all but scans of few
+// views), else an allocation in *own, which the caller frees. Two allocations and
+// releases a call took longer than the projections of small scans.
+int Session::volume_scratch(float **vol, float **own)
+{
+    *own = nullptr;
+    size_t acc = 0;
+    if (n_vox > 2 * n_sino && dalloc(own, n_vox, &acc)) return -1;
+    *vol = *own ? *own : reinterpret_cast<float *>(d_acc);
+    return 0;
+}
+
 int Session::forward_project(const float *obj, float *sino)
 {
     const Geom &g = hs.g;
-    float *d_obj = nullptr, *d_out = nullptr;
-    size_t acc = 0;
-    if (dalloc(&d_obj, n_vox, &acc) || dalloc(&d_out, n_sino, &acc)) {
-        if (d_obj) cudaFree(d_obj);
-        return -1;
-    }
-    cudaError_t e = cudaMemcpyAsync(d_tmp, obj, n_vox * sizeof(float), cudaMemcpyHostToDevice, st);
+    float *vol, *own;
+    if (volume_scratch(&vol, &own)) return -1;
+    cudaError_t e = cudaMemcpyAsync(vol, obj, n_vox * sizeof(float), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) {
-        launch_vol_to_zfast(d_tmp, d_obj, g.N_time, g.N_z, g.N_y, g.N_x, st);
-        launch_forward_project(g, d_table, d_view_first, d_obj, nullptr, d_acc, d_out, st);
+        // d_tmp holds the volume until the accumulation is done, then its result
+        launch_vol_to_zfast(vol, d_tmp, g.N_time, g.N_z, g.N_y, g.N_x, st);
+        launch_forward_project(g, d_table, d_view_first, d_tmp, nullptr, d_acc, d_tmp, st);
     }
     if (e == cudaSuccess) e = cudaGetLastError();
-    if (e == cudaSuccess) e = cudaMemcpyAsync(sino, d_out, n_sino * sizeof(float), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(sino, d_tmp, n_sino * sizeof(float), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(d_obj);
-    cudaFree(d_out);
+    if (own) cudaFree(own);
     if (e != cudaSuccess) return fail("forward projection failed: %s", cudaGetErrorString(e));
     return 0;
 }
@@ -643,22 +652,19 @@ int Session::forward_project(const float *obj, float *sino)
 int Session::back_project(const float *sino, float *obj)
 {
     const Geom &g = hs.g;
-    float *d_s = nullptr, *d_o = nullptr;
-    size_t acc = 0;
-    if (dalloc(&d_s, n_sino, &acc) || dalloc(&d_o, n_vox, &acc)) {
-        if (d_s) cudaFree(d_s);
-        return -1;
-    }
+    float *vol, *own;
+    if (volume_scratch(&vol, &own)) return -1;
+    // d_acc holds the sinogram until it is projected into d_tmp, then (as vol) the result
+    float *d_s = reinterpret_cast<float *>(d_acc);
     cudaError_t e = cudaMemcpyAsync(d_s, sino, n_sino * sizeof(float), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) launch_back_project(g, d_table, d_view_first, d_s, d_o, st);
+    if (e == cudaSuccess) launch_back_project(g, d_table, d_view_first, d_s, d_tmp, st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e == cudaSuccess) {
-        launch_zfast_to_vol(d_o, d_tmp, g.N_time, g.N_z, g.N_y, g.N_x, st);
-        e = cudaMemcpyAsync(obj, d_tmp, n_vox * sizeof(float), cudaMemcpyDeviceToHost, st);
+        launch_zfast_to_vol(d_tmp, vol, g.N_time, g.N_z, g.N_y, g.N_x, st);
+        e = cudaMemcpyAsync(obj, vol, n_vox * sizeof(float), cudaMemcpyDeviceToHost, st);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(d_s);
-    cudaFree(d_o);
+    if (own) cudaFree(own);
     if (e != cudaSuccess) return fail("back projection failed: %s", cudaGetErrorString(e));
     return 0;
 }
@@ -667,15 +673,14 @@ int Session::fbp(float *obj)
 {
     const Geom &g = hs.g;
     if (!fbp_supported(g)) return fail("FBP: %d channels x %d rows per view exceed the filter's shared memory", g.N_r, g.N_t);
-    float *d_o = nullptr;
-    size_t acc = 0;
-    if (dalloc(&d_o, n_vox, &acc)) return -1;
-    launch_fbp(g, d_table, d_view_first, d_y, d_tmp, d_o, st);
-    launch_zfast_to_vol(d_o, d_tmp, g.N_time, g.N_z, g.N_y, g.N_x, st);
+    float *vol, *own;
+    if (volume_scratch(&vol, &own)) return -1;
+    launch_fbp(g, d_table, d_view_first, d_y, d_tmp, vol, st);
+    launch_zfast_to_vol(vol, d_tmp, g.N_time, g.N_z, g.N_y, g.N_x, st);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(obj, d_tmp, n_vox * sizeof(float), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(d_o);
+    if (own) cudaFree(own);
     if (e != cudaSuccess) return fail("filtered back-projection failed: %s", cudaGetErrorString(e));
     return 0;
 }
