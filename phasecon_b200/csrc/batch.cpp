@@ -46,7 +46,6 @@ struct Batch {
         int2 *d_map = nullptr;  // interleaved (problem, item) per queue position
         int map_cap = 0, total = 0;
         int n = 0, grid = 0;
-        int smem = 0;           // dynamic shared memory of the class's launches
     } cls[2];
     static constexpr int kPhases = 16;  // K x K colours, K <= 4
     unsigned int *d_queue = nullptr;  // [class][phase]
@@ -146,7 +145,6 @@ int Batch::build_descs()
         if (!c.n) continue;
         std::vector<BatchDesc> h(c.n);
         std::vector<int> items(c.n);
-        c.smem = 0;
         for (int a = 0; a < c.n; a++) {
             Session &s = *m[c.idx[a]];
             BatchDesc &d = h[a];
@@ -163,8 +161,6 @@ int Batch::build_descs()
             d.L.colors_k = colors;
             d.L.perm = spread_multiplier(sv_slots(d.g.N_x, d.g.N_y, sv, colors));
             d.K = make_icd_const(s.hs.g);
-            batch_plan(d.g, d.L, c.vec);
-            c.smem = std::max(c.smem, d.L.shared_bytes);
             d.table = s.d_table;
             d.view_first = s.d_view_first;
             d.mask = s.d_mask;
@@ -196,7 +192,7 @@ int Batch::build_descs()
         }
         BCK(cudaMemcpyAsync(c.d_desc, h.data(), c.n * sizeof(BatchDesc), cudaMemcpyHostToDevice, st));
         BCK(cudaMemcpyAsync(c.d_map, map.data(), c.total * sizeof(int2), cudaMemcpyHostToDevice, st));
-        c.grid = (int)std::min<long long>(batch_grid(c.vec, warps, c.smem), grid_cap(c, sv, colors));
+        c.grid = (int)std::min<long long>(batch_grid(c.vec, warps), grid_cap(c, sv, colors));
     }
     BCK(cudaStreamSynchronize(st));
     return 0;
@@ -237,10 +233,9 @@ void Batch::enqueue_iteration(bool refresh)
             cudaStreamWaitEvent(st2, ev_fork, 0);
         }
         if (cls[0].n)
-            launch_icd_batch(4, warps, cls[0].grid, cls[0].smem, cls[0].d_desc, cls[0].d_map, cls[0].total, ph, d_queue + ph,
-                             st);
+            launch_icd_batch(4, warps, cls[0].grid, cls[0].d_desc, cls[0].d_map, cls[0].total, ph, d_queue + ph, st);
         if (cls[1].n)
-            launch_icd_batch(2, warps, cls[1].grid, cls[1].smem, cls[1].d_desc, cls[1].d_map, cls[1].total, ph,
+            launch_icd_batch(2, warps, cls[1].grid, cls[1].d_desc, cls[1].d_map, cls[1].total, ph,
                              d_queue + kPhases + ph, both ? st2 : st);
         if (both) {
             cudaEventRecord(ev_join, st2);

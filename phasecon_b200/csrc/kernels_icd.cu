@@ -22,21 +22,23 @@
 // time and visits its voxel columns one
 // after another in a seeded random order (the counterpart of
 // randomly_select_x_y, XT_ICD_update.c:499-531). For one column all warps
-// cooperate, with three CTA barriers per column:
+// cooperate, with two CTA barriers per column:
 //   1. neighbourhood: the 8 in-plane neighbour columns and the 2 temporal
 //      neighbours are split over the warps; each lane owns one slice z and
 //      accumulates the qGGMRF surrogate terms b = w rho'(d)/d of those
-//      neighbours (XT_ICD_update.c:140-172); a block-wide OR decides whether
-//      any slice escapes zero skipping (XT_VoxUpdate.c:238-261);
-//   2. theta: the column's views are split over warps; a lane owns one
-//      detector row t and accumulates theta1 = -sum a w e and theta2 =
-//      sum a^2 w over the column's A entries (a = A value x delta_t,
-//      XT_VoxUpdate.c:56-85) -- reads of e[view][r][0..N_t) are coalesced,
-//      and four views' records and entries are in flight at once;
+//      neighbours (XT_ICD_update.c:140-172), read from a tile of the SV and its
+//      surroundings in shared memory where it fits; whether any slice escapes zero
+//      skipping (XT_VoxUpdate.c:238-261) is decided from the same reads;
+//   2. theta: the column's A entries lie in lists in shared memory, one per warp
+//      and view group, unpacked from the records while the column before was
+//      solved; a lane owns VEC consecutive detector rows and accumulates theta1 =
+//      -sum a w e and theta2 = sum a^2 w over its list (a = A value x delta_t,
+//      XT_VoxUpdate.c:56-85) in packed FP32 arithmetic, a batch of up to 8
+//      entries' e and w in flight at once;
 //   3. solve: warp 0 sums the partials, then updates even slices and odd
 //      slices in turn (their only mutual coupling is the in-column z +- 1
 //      prior pair), x <- V + alpha (u - V);
-//   4. apply: e[view][r][t] -= a dx(slice of t) with atomic adds.
+//   4. apply: e[view][r][t] -= a dx(slice of t) with vector reductions.
 // All arithmetic is FP32; the host refreshes e in FP64 periodically.
 #include <mutex>
 #include <vector>
@@ -1051,6 +1053,8 @@ IcdConst make_icd_const(const Geom &g)
     K.ct = (float)g.c_t;
     K.qocs = (float)(g.q / g.c_s);
     K.qoct = (float)(g.q / g.c_t);
+    K.bs0 = (float)(g.q / (g.sigma_s_q * g.c_s));
+    K.bt0 = (float)(g.q / (g.sigma_t_q * g.c_t));
     K.alpha = (float)g.alpha;
     K.dt = (float)g.delta_t;
     K.huber_T = (float)g.huber_T;
@@ -1073,118 +1077,6 @@ void launch_icd_phase(const Geom &g, const IcdLaunch &L, const uint32_t *d_table
     const bool b8 = L.unroll > 0 ? L.unroll >= 2 : most > 4;
     const auto launch = v4 ? (b8 ? launch_vec<4, 8> : launch_vec<4, 4>) : (b8 ? launch_vec<2, 8> : launch_vec<2, 4>);
     launch(g, L, K, d_table, d_view_first, d_mask, d_x, d_err, d_w, d_mag, d_stats, d_queue, st);
-}
-
-// ---------------------------------------------------------------------------------------------
-// Many independent problems in one persistent launch per colour phase. The
-// queue runs over the SV items of every problem of the launch, interleaved in
-// proportion to each problem's item count (item_map[] gives the problem and
-// its item), so the CTAs working at any moment spread over the problems; a
-// CTA keeps the descriptor of its current problem in shared memory and
-// reloads it when its next item belongs to another problem. Problems of one
-// launch share the record width and the detector-row vector width (template
-// parameter).
-//
-// 64 registers, four entries in flight, entry lists unpacked from global memory:
-// eight CTAs of four warps stay on an SM, as many super-voxels in flight as the
-// convergence bound allows. That number is part of the method here: updates that
-// run at once act as extra over-relaxation, which speeds the slow modes up until
-// it diverges. The staged sweep with its tile is faster per iteration (8.0 against
-// 10.6 ms on 12 problems, 16.1 before) but keeps only three CTAs on an SM, and a
-// 256 x 256 x 8 problem of 129 views was then at twice the cost after 16 iterations.
-template <int VEC>
-__global__ void __launch_bounds__(kMaxWarps * 32, 4) icd_batch_kernel(const BatchDesc *__restrict__ descs,
-                                                                      const int2 *__restrict__ item_map, int total,
-                                                                      int phase, unsigned int *__restrict__ queue)
-{
-    __shared__ IcdSmem S;
-    __shared__ __align__(16) BatchDesc P;
-    extern __shared__ __align__(16) uint32_t s_dyn[];
-    int cur = -1;
-    IcdCount cnt{};
-    init_copies(S);
-    for (;;) {
-        __syncthreads();
-        if (threadIdx.x == 0) S.item = (int)atomicAdd(queue, 1u);
-        __syncthreads();
-        const int item = S.item;
-        if (item >= total) break;
-        const int2 pm = item_map[item];  // (problem, item of that problem)
-        if (pm.x != cur) {                // uniform
-            if (cur >= 0) flush_counts(cnt, P.stats);
-            __syncthreads();
-            const int4 *src = reinterpret_cast<const int4 *>(descs + pm.x);
-            int4 *dst = reinterpret_cast<int4 *>(&P);
-            for (int i = threadIdx.x; i < (int)(sizeof(BatchDesc) / sizeof(int4)); i += blockDim.x) dst[i] = src[i];
-            __syncthreads();
-            cur = pm.x;
-        }
-        if (!P.active) continue;
-        const int K = P.L.colors_k;
-        const int hx = (P.L.n_sv_x + K - 1) / K, slots = hx * ((P.L.n_sv_y + K - 1) / K);
-        const int f = pm.y % P.g.N_time;
-        const int rem = (int)((long long)(pm.y / P.g.N_time) * P.L.perm % slots);
-        const int color = (phase + f) % (K * K);
-        const int sx = K * (rem % hx) + color % K;
-        const int sy = K * (rem / hx) + color / K;
-        if (sx >= P.L.n_sv_x || sy >= P.L.n_sv_y) continue;
-        icd_update_sv<VEC, false, false, 2, 4>(P.g, P.L, P.K, P.table, P.view_first, P.mask, P.x, P.err, P.w, P.mag, f, sx, sy,
-                                               S, cnt, s_dyn);
-    }
-    if (cur >= 0) flush_counts(cnt, P.stats);
-}
-
-// Before an iteration: advance every problem's iteration number and clear its counters.
-__global__ void batch_begin_iteration(BatchDesc *descs, int n)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    descs[i].L.iter += 1;
-    *descs[i].stats = IcdStats{};
-}
-
-// After an iteration: accumulate the updates and stop problems whose
-// convergence statistic 100 sum|dx| / sum|x| fell below their threshold after
-// the first iteration (XT_ICD_update.c:1083-1090).
-__global__ void batch_end_iteration(BatchDesc *descs, int n)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || !descs[i].active) return;
-    const IcdStats s = *descs[i].stats;
-    descs[i].total_updates += s.updates;
-    descs[i].iters_done = descs[i].L.iter;
-    const double pct = s.sum_abs_x > 0 ? 100.0 * s.sum_abs_dx / s.sum_abs_x : 0.0;
-    descs[i].last_pct = pct;
-    if (descs[i].L.iter > 1 && pct < descs[i].convg_thresh) descs[i].active = 0;
-}
-
-void batch_plan(const Geom &g, IcdLaunch &L, int vec) { icd_plan_shared(g, L, vec, 4, ICD_PLAIN); }
-
-int batch_grid(int vec, int warps, int smem)
-{
-    int dev = 0, sms = 148, per_sm = 1;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, vec == 4 ? icd_batch_kernel<4> : icd_batch_kernel<2>, warps * 32,
-                                                  smem);
-    return sms * (per_sm > 0 ? per_sm : 1);
-}
-
-void launch_icd_batch(int vec, int warps, int grid, int smem, const BatchDesc *d_descs, const int2 *d_item_map, int total,
-                      int phase, unsigned int *d_queue, cudaStream_t st)
-{
-    if (vec == 4) icd_batch_kernel<4><<<grid, warps * 32, smem, st>>>(d_descs, d_item_map, total, phase, d_queue);
-    else icd_batch_kernel<2><<<grid, warps * 32, smem, st>>>(d_descs, d_item_map, total, phase, d_queue);
-}
-
-void launch_batch_begin(BatchDesc *d_descs, int n, cudaStream_t st)
-{
-    batch_begin_iteration<<<(n + 127) / 128, 128, 0, st>>>(d_descs, n);
-}
-
-void launch_batch_end(BatchDesc *d_descs, int n, cudaStream_t st)
-{
-    batch_end_iteration<<<(n + 127) / 128, 128, 0, st>>>(d_descs, n);
 }
 
 }  // namespace mbirgpu

@@ -128,7 +128,7 @@ struct IcdLaunch {
     int perm;             // queue order inside a frame: SV slot = (queue index * perm) mod slots
     int colors_k;         // K x K colour classes; phase p updates colour (p + frame) mod K^2
     long long max_ctas;   // cap on the persistent grid (sv_max_concurrent); 0 = none
-    int stage_records;    // prefetch each next column's A records into shared memory (cp.async)
+    int stage_records;    // copy each next column's A records into shared memory ahead of their use
     const int *iter_dev;  // if set, the iteration number is read here (graph-captured iterations)
     // optional explicit work list of the phase (non-homogeneous passes): items[i]
     // = frame << 22 | sv_y << 11 | sv_x, *n_items of them (device memory);
@@ -180,6 +180,7 @@ struct IcdConst {
     float q, qmp, cs, ct, alpha, dt;
     float issq, issqp, istq, istqp;  // reciprocals of the scale powers sigma^q, sigma^(q-p) (space, time)
     float qocs, qoct;                // q / c: the surrogate weight at a zero difference times sigma^q
+    float bs0, bt0;                  // the same over sigma^q
     float huber_T, huber_T2, huber_delta;  // T2: T^2 less a margin for rounding
     int huber;
 };
@@ -209,11 +210,9 @@ struct __align__(16) BatchDesc {
     int active;                        // 0 once converged: its items are skipped
     int iters_done;
 };
-// Shared-memory plan of one problem of a batched launch (fills L's fields),
-// the persistent grid, the launch.
-void batch_plan(const Geom &g, IcdLaunch &L, int vec);
-int batch_grid(int vec, int warps, int smem);
-void launch_icd_batch(int vec, int warps, int grid, int smem, const BatchDesc *d_descs, const int2 *d_item_map, int total,
+// The persistent grid of a batched launch, and the launch.
+int batch_grid(int vec, int warps);
+void launch_icd_batch(int vec, int warps, int grid, const BatchDesc *d_descs, const int2 *d_item_map, int total,
                       int phase, unsigned int *d_queue, cudaStream_t st);
 // Stability of concurrent super-voxel updates: CTAs update different columns
 // at the same time, and columns of one frame on a common ray couple like a

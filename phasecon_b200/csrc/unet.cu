@@ -20,8 +20,9 @@
 //   data grad the same kernel on the output gradient with the weights
 //             flipped in space and transposed in channels;
 //   weight grad dw[tap][ci][co] = sum_v in[v + off(tap)][ci] g[v][co]
-//             (M = ci, N = co, K = voxels) over the same tiles, all 27 taps
-//             from one staged halo, FP32 atomics once per CTA.
+//             (M = ci, N = co, K = voxels): asynchronous copies bring the
+//             tiles, ldmatrix.trans turns them, all 27 taps from one staged
+//             halo, FP32 atomics once per CTA.
 #include <cuda_bf16.h>
 
 #include <algorithm>
