@@ -60,8 +60,8 @@ typedef struct {
     int32_t refresh_every;   /* FP64 recomputation of e = y - Ax every n iterations, default 8 */
     int32_t sv_size;         /* super-voxel edge in voxel columns; 0 = by rule or autotuned */
     int32_t cta_warps;       /* warps cooperating on one voxel column; 0 = by rule or autotuned */
-    int32_t icd_unroll;      /* views whose A records and sinogram entries one lane keeps in flight
-                                (1, 2 or 4); 0 = autotuned */
+    int32_t icd_unroll;      /* sinogram entries one lane keeps in flight: 1 for four, 2 or more for
+                                eight; 0 = by rule */
     uint64_t seed;           /* voxel-order seed */
     int32_t nhicd_passes;    /* non-homogeneous ICD (XT_ICD_update.c:1007-1047, XT_NHICD.c:164-216):
                                 from iteration 2, after the full sweep, n passes each re-update the
@@ -81,8 +81,9 @@ typedef struct {
     int32_t nh_work_lists;   /* 1 (default): those passes visit only super-voxels holding selected
                                 columns, the ones with the most first; 0: every super-voxel */
     int32_t autotune;        /* 0 (default): the schedule fields left at 0 follow a fixed rule of
-                                the problem's shape (super-voxels 4 x 4, K = 2, 4 warps per column
-                                when a frame has >= 64 views, else 2), so the same inputs give the
+                                the problem's shape (super-voxels 4 x 4, K = 2, 2 to 8 warps per
+                                column, fewer the more super-voxels are in flight and the fewer
+                                entries a column has), so the same inputs give the
                                 same schedule and the same image on every run; 1: a single
                                 session measures the candidate schedules on its own problem and
                                 keeps the fastest (timing-dependent); batches always measure */
