@@ -426,7 +426,7 @@ __device__ __forceinline__ unsigned mod_small(uint64_t h, unsigned d)
 // kTile: the neighbours' values are read from the tile in shared memory
 // (stage_tile), else from x;
 // kHuber: 0 the quadratic data term, 1 the generalised Huber one
-// (XT_VoxUpdate.c:68-82), 2 decided per problem at run time (K.huber);
+// (XT_VoxUpdate.c:68-82);
 // kBatch: entries of a lane in flight together.
 //
 // A view's entries are read (theta) and reduced into (apply) by the same lane
@@ -676,7 +676,7 @@ __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L,
 #pragma unroll
                         for (int i = 0; i < VEC / 2; i++) {
                             f32x2 ww = w[u].p[i];
-                            if (kHuber == 1 || (kHuber == 2 && K.huber)) {
+                            if (kHuber) {
                                 float w0, w1, e0, e1;
                                 unpack2(ww, w0, w1);
                                 unpack2(e[u].p[i], e0, e1);

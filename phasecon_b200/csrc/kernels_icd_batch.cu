@@ -152,7 +152,7 @@ __device__ __forceinline__ void flush_counts(IcdCount &cnt, IcdStats *stats)
 // sinogram row offset `row0` within each A entry's row, views gfirst,
 // gfirst + gstride, ... of the column): theta1 = -sum a w e,
 // theta2 = sum a^2 w with a = A value x delta_t (XT_VoxUpdate.c:56-85).
-template <int KW, int kUnroll, int VEC, int kHuber>
+template <int KW, int kUnroll, int VEC>
 __device__ __forceinline__ void theta_pass(const IcdConst &K, const uint32_t *col_rec, const float *__restrict__ err,
                                            const float *__restrict__ wgt, int gfirst, int gstride, int nv, int RW,
                                            int NT, int row0, float (&th1)[VEC], float (&th2)[VEC])
@@ -182,7 +182,7 @@ __device__ __forceinline__ void theta_pass(const IcdConst &K, const uint32_t *co
 #pragma unroll
                     for (int i = 0; i < VEC; i++) {
                         float ww = wv[i];
-                        if (kHuber == 1 || (kHuber == 2 && K.huber)) {
+                        if (K.huber) {
                             const float sw = sqrtf(ww);
                             if (!(fabsf(ev[i] * sw) < K.huber_T)) ww = K.huber_T * K.huber_delta * sw / fabsf(ev[i]);
                         }
@@ -199,7 +199,7 @@ __device__ __forceinline__ void theta_pass(const IcdConst &K, const uint32_t *co
 // One column's theta: every lane's partial sums (theta_pass, when `run`),
 // folded over the view groups of the warp and stored by group 0 into the
 // warp's row of S.th1 / S.th2.
-template <int KW, int kUnroll, int VEC, int kHuber>
+template <int KW, int kUnroll, int VEC>
 __device__ __forceinline__ void theta_column(const IcdConst &K, const uint32_t *col_rec, const float *__restrict__ err,
                                              const float *__restrict__ wgt, int gfirst, int gstride, int nv, int RW,
                                              int NT, int row0, bool run, int lprp, int grp, int t0, int warp,
@@ -208,7 +208,7 @@ __device__ __forceinline__ void theta_column(const IcdConst &K, const uint32_t *
     float th1[VEC], th2[VEC];
 #pragma unroll
     for (int i = 0; i < VEC; i++) th1[i] = th2[i] = 0.0f;
-    if (run) theta_pass<KW, kUnroll, VEC, kHuber>(K, col_rec, err, wgt, gfirst, gstride, nv, RW, NT, row0, th1, th2);
+    if (run) theta_pass<KW, kUnroll, VEC>(K, col_rec, err, wgt, gfirst, gstride, nv, RW, NT, row0, th1, th2);
     for (int off = lprp; off < 32; off <<= 1) {
 #pragma unroll
         for (int i = 0; i < VEC; i++) {
@@ -231,9 +231,9 @@ __device__ __forceinline__ void theta_column(const IcdConst &K, const uint32_t *
 // KW: 16-byte words per A record (1, 2, 3 for voxel scale 1, 2, 4);
 // kUnroll: views whose records and sinogram entries are in flight together;
 // VEC: consecutive detector rows one lane owns (4 when N_t % 4 == 0, else 2);
-// kHuber: 0 the quadratic data term, 1 the generalised Huber one
-// (XT_VoxUpdate.c:68-82), 2 decided per problem at run time (K.huber).
-template <int KW, int kUnroll, int VEC, int kHuber>
+// The data term (quadratic or generalised Huber, XT_VoxUpdate.c:68-82) is decided per
+// problem at run time (K.huber).
+template <int KW, int kUnroll, int VEC>
 __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L, const IcdConst &K,
                                               const uint32_t *__restrict__ table,
                                               const int32_t *__restrict__ view_first,
@@ -379,7 +379,7 @@ __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L,
             // a thread whose wait gave up reads no record (their headers address
             // the sinogram); the CTA leaves after the barrier
             if (sure)
-                theta_column<KW, kUnroll, VEC, kHuber>(K, col_rec, err, wgt, gfirst, gstride, nv, RW, NT,
+                theta_column<KW, kUnroll, VEC>(K, col_rec, err, wgt, gfirst, gstride, nv, RW, NT,
                                                                rbase + t0, row_ok, lprp, grp, t0, warp, S);
             const int any_active = __syncthreads_or(active_pred);
             if (!any_active) {
@@ -388,7 +388,7 @@ __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L,
                 continue;  // uniform across the CTA
             }
             if (!sure) {  // uniform across the CTA
-                theta_column<KW, kUnroll, VEC, kHuber>(K, col_rec, err, wgt, gfirst, gstride, nv, RW, NT,
+                theta_column<KW, kUnroll, VEC>(K, col_rec, err, wgt, gfirst, gstride, nv, RW, NT,
                                                                rbase + t0, row_ok, lprp, grp, t0, warp, S);
                 __syncthreads();
             }
@@ -561,7 +561,7 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 4) icd_batch_kernel(const Batc
         const int sx = K * (rem % hx) + color % K;
         const int sy = K * (rem / hx) + color / K;
         if (sx >= P.L.n_sv_x || sy >= P.L.n_sv_y) continue;
-        icd_update_sv<KW, kUnroll, VEC, 2>(P.g, P.L, P.K, P.table, P.view_first, P.mask, P.x, P.err, P.w, P.mag,
+        icd_update_sv<KW, kUnroll, VEC>(P.g, P.L, P.K, P.table, P.view_first, P.mask, P.x, P.err, P.w, P.mag,
                                                f, sx, sy, S, cnt);
     }
     if (cur >= 0) flush_counts(cnt, P.stats);
