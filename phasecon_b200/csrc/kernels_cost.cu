@@ -83,9 +83,13 @@ __device__ __forceinline__ double exp2_of(double y, const PowTables &T)
     return __hiloint2double(__double2hiint(v) + ((n >> 6) << 20), __double2loint(v));
 }
 
+// The largest exponent whose powers stay in exp2_of's range: |d| is 2^-149 to 2^128.
+constexpr double kMaxFastQ = 6.5;
+
 // sum += |d|^q / (c + |d|^(q-p) / sqp), branch-free so that several run at once. A
 // zero difference adds nothing; bad is set where the fast form does not hold (an
-// infinite or NaN difference, a denominator outside 2^-100 .. 2^100).
+// infinite or NaN difference, a denominator outside 2^-100 .. 2^100; the caller sets it
+// for exponents past kMaxFastQ).
 __device__ __forceinline__ void add_potential(double &sum, bool &bad, float d, double q, double qmp, double inv_sqp,
                                               double c, const PowTables &T)
 {
@@ -179,7 +183,7 @@ __global__ void __launch_bounds__(kCostThreads) cost_partials_kernel(Geom g, con
             for (int i = 0; i < 14; i++) any |= d[i] != 0.0f;
             if (!any) continue;
             double s[4] = {0, 0, 0, 0};
-            bool bad = false;
+            bool bad = !(g.q <= kMaxFastQ);
 #pragma unroll
             for (int i = 0; i < 14; i++)
                 add_potential(s[i < 3 ? 0 : i < 9 ? 1 : i < 13 ? 2 : 3], bad, d[i], g.q, qmp, i < 13 ? inv_ssqp : inv_stqp,
