@@ -352,8 +352,8 @@ __global__ void __launch_bounds__(256, 3) back_project_kernel(Geom g, int L, int
     }
 }
 
-// Back projection over longer records (coarse voxel scales) and z scales that are no
-// power of two: lane = detector row, one warp per column and chunk.
+// Back projection over longer records (coarse voxel scales): lane = detector row, one
+// warp per column and chunk.
 __global__ void back_project_wide_kernel(Geom g, const uint32_t *__restrict__ table,
                                          const int32_t *__restrict__ view_first, const float *__restrict__ sino,
                                          float *__restrict__ out)
@@ -386,11 +386,46 @@ __global__ void back_project_wide_kernel(Geom g, const uint32_t *__restrict__ ta
         out[((size_t)f * nxy + c) * g.N_z + t / g.z_overlap] = (float)acc;
 }
 
+// Back projection over z scales that do not divide a chunk of rows (no power of two, or
+// above 32): lane = slice, which adds up its own z_overlap rows; one warp per column and
+// 32 slices.
+__global__ void back_project_slices_kernel(Geom g, const uint32_t *__restrict__ table,
+                                           const int32_t *__restrict__ view_first, const float *__restrict__ sino,
+                                           float *__restrict__ out)
+{
+    const int nxy = g.N_x * g.N_y;
+    const int n_chunks = (g.N_z + 31) / 32;
+    const long long gw = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
+    if (gw >= (long long)g.N_time * nxy * n_chunks) return;
+    const int z = (int)(gw % n_chunks) * 32 + (threadIdx.x & 31);
+    if (z >= g.N_z) return;
+    const long long fc = gw / n_chunks;
+    const int f = (int)(fc / nxy), c = (int)(fc - (long long)f * nxy);
+    const int fv0 = view_first[f], nv = view_first[f + 1] - fv0;
+    const uint32_t *rec = table + ((size_t)fv0 * nxy + (size_t)c * nv) * g.rec_words;
+    double acc = 0.0;
+    for (int v = 0; v < nv; v++, rec += g.rec_words) {
+        const uint32_t hdr = __ldg(rec);
+        const int cnt = hdr >> 24;
+        const float *p = sino + (size_t)(hdr & 0xFFFFFF) * g.N_t + (size_t)z * g.z_overlap;
+        for (int q = 0; q < cnt; q++, p += g.N_t) {
+            const double a = (double)__uint_as_float(__ldg(rec + 1 + q));
+            for (int r = 0; r < g.z_overlap; r++) acc += a * (double)__ldg(p + r);
+        }
+    }
+    out[((size_t)f * nxy + c) * g.N_z + z] = (float)acc;
+}
+
 void launch_back_project(const Geom &g, const uint32_t *d_table, const int32_t *d_view_first,
                          const float *d_sino, float *d_x, cudaStream_t st)
 {
-    const int zo = g.z_overlap, chunks = (g.N_t + kRowChunk - 1) / kRowChunk;
-    if (g.rec_words != 4 || (zo & (zo - 1)) || zo > kRowChunk) {
+    const int chunks = (g.N_t + kRowChunk - 1) / kRowChunk;
+    if (kRowChunk % g.z_overlap) {
+        const long long warps = (long long)g.N_time * g.N_x * g.N_y * ((g.N_z + 31) / 32);
+        back_project_slices_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(g, d_table, d_view_first, d_sino, d_x);
+        return;
+    }
+    if (g.rec_words != 4) {
         const long long warps = (long long)g.N_time * g.N_x * g.N_y * chunks;
         back_project_wide_kernel<<<(unsigned)((warps + 7) / 8), 256, 0, st>>>(g, d_table, d_view_first, d_sino, d_x);
         return;
