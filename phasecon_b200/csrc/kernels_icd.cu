@@ -427,12 +427,13 @@ __device__ __forceinline__ unsigned mod_small(uint64_t h, unsigned d)
 // (stage_tile), else from x;
 // kHuber: 0 the quadratic data term, 1 the generalised Huber one
 // (XT_VoxUpdate.c:68-82);
-// kBatch: entries of a lane in flight together.
+// kBatch: entries of a lane in flight together;
+// kAnyZ: slices' rows need not divide a chunk of 32 (below).
 //
 // A view's entries are read (theta) and reduced into (apply) by the same lane
 // for every column of the SV, so no barrier is needed between one column's
 // apply pass and the next one's theta loads.
-template <int VEC, bool kStaged, bool kTile, int kHuber, int kBatch>
+template <int VEC, bool kStaged, bool kTile, int kHuber, int kBatch, bool kAnyZ>
 __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L, const IcdConst &K,
                                               const uint32_t *__restrict__ table,
                                               const int32_t *__restrict__ view_first,
@@ -451,8 +452,14 @@ __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L,
     // A voxel column is updated in chunks of at most 32 detector rows (32 / MZ
     // voxel slices, one per lane of warp 0); chunk k covers rows [32k, 32k + 32)
     // and slices [k CZ, k CZ + CZ). Columns of up to 32 rows are one chunk.
-    const int CT = NT < 32 ? NT : 32, CZ = CT / MZ;
-    const int n_chunks = (NT + 31) / 32;
+    // kAnyZ (taller columns whose slices' rows, MZ, do not divide 32): a chunk is the
+    // rows of its CZ slices (of one slice where MZ > 32), from wherever these begin.
+    // Lanes hold two aligned rows (VEC 2), so the chunk is gone through in blocks of 32
+    // rows from the aligned row at or before its first one; rows outside it count as
+    // zero. MZ <= 31 gives one block (CZ MZ <= 31 and at most one row before them).
+    static_assert(!kAnyZ || (VEC == 2 && !kStaged && !kTile), "any z scale: two rows a lane, lists from global memory");
+    const int CT = NT < 32 ? NT : 32, CZ = kAnyZ ? max(1, 32 / MZ) : CT / MZ;
+    const int n_chunks = kAnyZ ? (NZ + CZ - 1) / CZ : (NT + 31) / 32;
 
     // lane -> (view group, run of VEC detector rows) for the theta / apply passes
     const int lprp = icd_lanes_per_row(NT, VEC);
@@ -560,9 +567,18 @@ __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L,
         for (int ch = 0; ch < n_chunks; ch++) {
             const int z0 = ch * CZ;                                  // first slice of the chunk
             const int cz = NZ - z0 < CZ ? NZ - z0 : CZ;              // slices in the chunk
-            const int rbase = ch * 32;                               // first detector row of the chunk
-            const bool row_ok = tq < cz * MZ / VEC;
-            const unsigned rows0 = (unsigned)(rbase + t0);           // this lane's rows within an entry
+            const int first_row = kAnyZ ? z0 * MZ : ch * 32, end_row = first_row + cz * MZ;  // the chunk's rows
+            const int rbase = kAnyZ ? first_row & ~(VEC - 1) : first_row;  // first row of its first block
+            int rb = rbase;                                                // of the current block
+            bool row_ok = kAnyZ ? rb + t0 < end_row : tq < cz * MZ / VEC;
+            unsigned rows0 = (unsigned)(rb + t0);  // this lane's rows within an entry
+            // (kAnyZ) go on to the chunk's next block of rows
+            auto next_rows = [&]() {
+                rb += 32;
+                row_ok = rb + t0 < end_row;
+                rows0 = (unsigned)(rb + t0);
+                return rb < end_row;
+            };
             bool active = ci >= 0;
             float V = 0.0f;
             int vb = 0;
@@ -592,146 +608,162 @@ __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L,
                 if (!kStaged) next_block();
                 int n_ent = row_ok ? (int)ent[0].x : 0, n_warp = (int)ent[0].y, i0 = 0;
                 bool first = true;
-                for (;;) {
-                    // entries i0 .. i0 + kBatch - 1: all loads in flight together
+                for (;;) {  // once; kAnyZ: the chunk's blocks of rows
+                    for (;;) {
+                        // entries i0 .. i0 + kBatch - 1: all loads in flight together
 #pragma unroll
-                    for (int u = 0; u < kBatch; u++) {
-                        const uint2 en = ent[1 + i0 + u];
-                        const unsigned off = en.x + rows0;
-                        na[u] = __uint_as_float(en.y);
-                        load_entry(e[u], w[u], err + off, wgt + off, i0 + u, n_ent);
-                    }
-                    // ---- 1. neighbourhood, while the first batch arrives (sources
-                    //         split over warps and lane groups) ------------------------
-                    if (first) {
-                        first = false;
-                        float num = 0.0f, den = 0.0f, top = 0.0f;  // top: the largest neighbour, or 0
-                        const bool zm = z > 0, zn = z + 1 < NZ;
-                        for (int s0 = sfirst; s0 < 8; s0 += sstride) {  // in-plane; uniform over the warp
-                            const int s = min(s0 + sub, 7);
-                            int dy, dx;
-                            source_step(s, dy, dx);
-                            const bool ok = zl && s0 + sub < 8 && ((inside >> s) & 1), side = dy == 0 || dx == 0;
-                            const float *src = cb + (ptrdiff_t)((dy * (kTile ? TW : NX) + dx) * NZ);
-                            float n[3], d[3], fl[3], cf[3];
-                            // (in the tile every address read exists: values outside the
-                            // object are dropped after the load, without a branch)
-                            const float nm = kTile || (ok && zm) ? src[z - 1] : 0.0f;
-                            const float n0 = kTile || ok ? src[z] : 0.0f;
-                            const float np = kTile || (ok && zn) ? src[z + 1] : 0.0f;
-                            n[0] = ok && zm ? nm : 0.0f;
-                            n[1] = ok ? n0 : 0.0f;
-                            n[2] = ok && zn ? np : 0.0f;
-                            const float fo = side ? f2 : f3;
-                            fl[0] = ok && zm ? fo : 0.0f;
-                            fl[1] = ok ? (side ? f1 : f2) : 0.0f;
-                            fl[2] = ok && zn ? fo : 0.0f;
-#pragma unroll
-                            for (int i = 0; i < 3; i++) d[i] = V - n[i];
-                            qg_coef(d, fl, K.q, K.qmp, K.issqp, K.cs, K.qocs, cf);
-#pragma unroll
-                            for (int i = 0; i < 3; i++) {
-                                num += cf[i] * n[i];
-                                den += cf[i];
-                                top = fmaxf(top, n[i]);
-                            }
+                        for (int u = 0; u < kBatch; u++) {
+                            const uint2 en = ent[1 + i0 + u];
+                            const unsigned off = en.x + rows0;
+                            na[u] = __uint_as_float(en.y);
+                            load_entry(e[u], w[u], err + off, wgt + off, i0 + u, n_ent);
                         }
-                        // temporal (the same source for every lane of a lane group)
-                        for (int t0_ = ts - sub; t0_ < 2 && t0_ >= 0; t0_ += sstride) {
-                            const int t = min(t0_ + sub, 1);
-                            const bool ok = zl && t0_ + sub < 2 && ((inside >> (8 + t)) & 1);
-                            const float *src = kTile ? cb + (t + 1) * TW * TW * NZ
-                                                     : cb + (t == 0 ? -(ptrdiff_t)nxy : (ptrdiff_t)nxy) * NZ;
-                            const float n0 = kTile || ok ? src[z] : 0.0f;
-                            const float n[1] = {ok ? n0 : 0.0f}, d[1] = {V - n[0]}, fl[1] = {ok ? K.tf * K.istq : 0.0f};
-                            float cf[1];
-                            qg_coef(d, fl, K.q, K.qmp, K.istqp, K.ct, K.qoct, cf);
-                            num += cf[0] * n[0];
-                            den += cf[0];
-                            top = fmaxf(top, n[0]);
-                        }
-                        unsigned pw = __ballot_sync(0xffffffffu, top > 0.0f);
-                        for (int off = zp; off < 32; off <<= 1) {
-                            num += __shfl_xor_sync(0xffffffffu, num, off);
-                            den += __shfl_xor_sync(0xffffffffu, den, off);
-                            pw |= pw >> off;
-                        }
-                        if (sub == 0) S.nd[warp][zlane] = make_float2(num, den);
-                        if (lane == 0) S.pos[warp] = pw & (0xffffffffu >> (32 - zp));
-                        // a column that may be inactive (all of it zero) needs the
-                        // neighbours' verdict first (uniform: every warp read the column)
-                        if (!sure) {
-                            __syncthreads();
-                            unsigned any = 0;
-                            for (int q = 0; q < W; q++) any |= S.pos[q];
-                            active = any != 0;
-                            if (!active) break;
-                        }
-                    }
-                    // ---- 2. theta1 = -sum a w e, theta2 = sum a^2 w over the column's
-                    //         entries (XT_VoxUpdate.c:56-85) ---------------------------
+                        // ---- 1. neighbourhood, while the first batch arrives (sources
+                        //         split over warps and lane groups) ------------------------
+                        if (first) {
+                            first = false;
+                            float num = 0.0f, den = 0.0f, top = 0.0f;  // top: the largest neighbour, or 0
+                            const bool zm = z > 0, zn = z + 1 < NZ;
+                            for (int s0 = sfirst; s0 < 8; s0 += sstride) {  // in-plane; uniform over the warp
+                                const int s = min(s0 + sub, 7);
+                                int dy, dx;
+                                source_step(s, dy, dx);
+                                const bool ok = zl && s0 + sub < 8 && ((inside >> s) & 1), side = dy == 0 || dx == 0;
+                                const float *src = cb + (ptrdiff_t)((dy * (kTile ? TW : NX) + dx) * NZ);
+                                float n[3], d[3], fl[3], cf[3];
+                                // (in the tile every address read exists: values outside the
+                                // object are dropped after the load, without a branch)
+                                const float nm = kTile || (ok && zm) ? src[z - 1] : 0.0f;
+                                const float n0 = kTile || ok ? src[z] : 0.0f;
+                                const float np = kTile || (ok && zn) ? src[z + 1] : 0.0f;
+                                n[0] = ok && zm ? nm : 0.0f;
+                                n[1] = ok ? n0 : 0.0f;
+                                n[2] = ok && zn ? np : 0.0f;
+                                const float fo = side ? f2 : f3;
+                                fl[0] = ok && zm ? fo : 0.0f;
+                                fl[1] = ok ? (side ? f1 : f2) : 0.0f;
+                                fl[2] = ok && zn ? fo : 0.0f;
 #pragma unroll
-                    for (int u = 0; u < kBatch; u++) {
-                        const f32x2 a = pack2(na[u], na[u]);
+                                for (int i = 0; i < 3; i++) d[i] = V - n[i];
+                                qg_coef(d, fl, K.q, K.qmp, K.issqp, K.cs, K.qocs, cf);
 #pragma unroll
-                        for (int i = 0; i < VEC / 2; i++) {
-                            f32x2 ww = w[u].p[i];
-                            if (kHuber) {
-                                float w0, w1, e0, e1;
-                                unpack2(ww, w0, w1);
-                                unpack2(e[u].p[i], e0, e1);
-                                // |e sqrt(w)| >= T only if e^2 w >= T^2 up to rounding: most
-                                // entries need no square root
-                                if (!(e0 * e0 * w0 < K.huber_T2 && w0 >= 0.0f && e1 * e1 * w1 < K.huber_T2 && w1 >= 0.0f)) {
-                                    const float s0 = sqrtf(w0), s1 = sqrtf(w1);
-                                    if (!(fabsf(e0 * s0) < K.huber_T)) w0 = K.huber_T * K.huber_delta * s0 / fabsf(e0);
-                                    if (!(fabsf(e1 * s1) < K.huber_T)) w1 = K.huber_T * K.huber_delta * s1 / fabsf(e1);
-                                    ww = pack2(w0, w1);
+                                for (int i = 0; i < 3; i++) {
+                                    num += cf[i] * n[i];
+                                    den += cf[i];
+                                    top = fmaxf(top, n[i]);
                                 }
                             }
-                            const f32x2 aw = mul2(a, ww);  // -a w
-                            t2[i] = fma2(a, aw, t2[i]);
-                            t1[i] = fma2(e[u].p[i], aw, t1[i]);
+                            // temporal (the same source for every lane of a lane group)
+                            for (int t0_ = ts - sub; t0_ < 2 && t0_ >= 0; t0_ += sstride) {
+                                const int t = min(t0_ + sub, 1);
+                                const bool ok = zl && t0_ + sub < 2 && ((inside >> (8 + t)) & 1);
+                                const float *src = kTile ? cb + (t + 1) * TW * TW * NZ
+                                                         : cb + (t == 0 ? -(ptrdiff_t)nxy : (ptrdiff_t)nxy) * NZ;
+                                const float n0 = kTile || ok ? src[z] : 0.0f;
+                                const float n[1] = {ok ? n0 : 0.0f}, d[1] = {V - n[0]}, fl[1] = {ok ? K.tf * K.istq : 0.0f};
+                                float cf[1];
+                                qg_coef(d, fl, K.q, K.qmp, K.istqp, K.ct, K.qoct, cf);
+                                num += cf[0] * n[0];
+                                den += cf[0];
+                                top = fmaxf(top, n[0]);
+                            }
+                            unsigned pw = __ballot_sync(0xffffffffu, top > 0.0f);
+                            for (int off = zp; off < 32; off <<= 1) {
+                                num += __shfl_xor_sync(0xffffffffu, num, off);
+                                den += __shfl_xor_sync(0xffffffffu, den, off);
+                                pw |= pw >> off;
+                            }
+                            if (sub == 0) S.nd[warp][zlane] = make_float2(num, den);
+                            if (lane == 0) S.pos[warp] = pw & (0xffffffffu >> (32 - zp));
+                            // a column that may be inactive (all of it zero) needs the
+                            // neighbours' verdict first (uniform: every warp read the column)
+                            if (!sure) {
+                                __syncthreads();
+                                unsigned any = 0;
+                                for (int q = 0; q < W; q++) any |= S.pos[q];
+                                active = any != 0;
+                                if (!active) break;
+                            }
+                        }
+                        // ---- 2. theta1 = -sum a w e, theta2 = sum a^2 w over the column's
+                        //         entries (XT_VoxUpdate.c:56-85) ---------------------------
+#pragma unroll
+                        for (int u = 0; u < kBatch; u++) {
+                            const f32x2 a = pack2(na[u], na[u]);
+#pragma unroll
+                            for (int i = 0; i < VEC / 2; i++) {
+                                f32x2 ww = w[u].p[i];
+                                if (kHuber) {
+                                    float w0, w1, e0, e1;
+                                    unpack2(ww, w0, w1);
+                                    unpack2(e[u].p[i], e0, e1);
+                                    // |e sqrt(w)| >= T only if e^2 w >= T^2 up to rounding: most
+                                    // entries need no square root
+                                    if (!(e0 * e0 * w0 < K.huber_T2 && w0 >= 0.0f && e1 * e1 * w1 < K.huber_T2 && w1 >= 0.0f)) {
+                                        const float s0 = sqrtf(w0), s1 = sqrtf(w1);
+                                        if (!(fabsf(e0 * s0) < K.huber_T)) w0 = K.huber_T * K.huber_delta * s0 / fabsf(e0);
+                                        if (!(fabsf(e1 * s1) < K.huber_T)) w1 = K.huber_T * K.huber_delta * s1 / fabsf(e1);
+                                        ww = pack2(w0, w1);
+                                    }
+                                }
+                                const f32x2 aw = mul2(a, ww);  // -a w
+                                t2[i] = fma2(a, aw, t2[i]);
+                                t1[i] = fma2(e[u].p[i], aw, t1[i]);
+                            }
+                        }
+                        i0 += kBatch;
+                        if (i0 >= n_warp) {  // uniform over the warp
+                            vb += L.block_views;
+                            if (kStaged || vb >= nv) break;
+                            next_block();
+                            n_ent = row_ok ? (int)ent[0].x : 0;
+                            n_warp = (int)ent[0].y;
+                            i0 = 0;
                         }
                     }
-                    i0 += kBatch;
-                    if (i0 >= n_warp) {  // uniform over the warp
-                        vb += L.block_views;
-                        if (kStaged || vb >= nv) break;
-                        next_block();
-                        n_ent = row_ok ? (int)ent[0].x : 0;
-                        n_warp = (int)ent[0].y;
-                        i0 = 0;
-                    }
-                }
-                if (active) {
-                    // sum over the warp's view groups: two groups share out their rows
-                    // until a lane holds one row, then add it up over the rest
-                    float a[VEC], b[VEC];
+                    if (active) {
+                        // sum over the warp's view groups: two groups share out their rows
+                        // until a lane holds one row, then add it up over the rest
+                        float a[VEC], b[VEC];
 #pragma unroll
-                    for (int i = 0; i < VEC / 2; i++) {
-                        unpack2(t1[i], a[2 * i], a[2 * i + 1]);
-                        unpack2(t2[i], b[2 * i], b[2 * i + 1]);
-                    }
-                    int row = t0, off = lprp;
-#pragma unroll
-                    for (int n = VEC / 2; n >= 1; n /= 2) {
-                        const bool up = (lane & off) != 0;
-#pragma unroll
-                        for (int i = 0; i < n; i++) {
-                            const float sa = up ? a[i] : a[n + i], sb = up ? b[i] : b[n + i];
-                            a[i] = (up ? a[n + i] : a[i]) + __shfl_xor_sync(0xffffffffu, sa, off);
-                            b[i] = (up ? b[n + i] : b[i]) + __shfl_xor_sync(0xffffffffu, sb, off);
+                        for (int i = 0; i < VEC / 2; i++) {
+                            unpack2(t1[i], a[2 * i], a[2 * i + 1]);
+                            unpack2(t2[i], b[2 * i], b[2 * i + 1]);
                         }
-                        row += up ? n : 0;
-                        off <<= 1;
+                        int row = t0, off = lprp;
+#pragma unroll
+                        for (int n = VEC / 2; n >= 1; n /= 2) {
+                            const bool up = (lane & off) != 0;
+#pragma unroll
+                            for (int i = 0; i < n; i++) {
+                                const float sa = up ? a[i] : a[n + i], sb = up ? b[i] : b[n + i];
+                                a[i] = (up ? a[n + i] : a[i]) + __shfl_xor_sync(0xffffffffu, sa, off);
+                                b[i] = (up ? b[n + i] : b[i]) + __shfl_xor_sync(0xffffffffu, sb, off);
+                            }
+                            row += up ? n : 0;
+                            off <<= 1;
+                        }
+                        const bool writes = lane < off && row_ok;
+                        for (; off < 32; off <<= 1) {
+                            a[0] += __shfl_xor_sync(0xffffffffu, a[0], off);
+                            b[0] += __shfl_xor_sync(0xffffffffu, b[0], off);
+                        }
+                        if (!kAnyZ) {
+                            if (writes) S.th[warp][row] = make_float2(a[0], b[0]);
+                        } else if (writes) {
+                            // rows outside the chunk are zero; a slice of several blocks adds
+                            // them up (the same lane holds a row of every block)
+                            const bool in = rb + row >= first_row && rb + row < end_row;
+                            const float2 sum = rb == rbase ? make_float2(0.0f, 0.0f) : S.th[warp][row];
+                            S.th[warp][row] = make_float2(sum.x + (in ? a[0] : 0.0f), sum.y + (in ? b[0] : 0.0f));
+                        }
                     }
-                    const bool writes = lane < off && row_ok;
-                    for (; off < 32; off <<= 1) {
-                        a[0] += __shfl_xor_sync(0xffffffffu, a[0], off);
-                        b[0] += __shfl_xor_sync(0xffffffffu, b[0], off);
-                    }
-                    if (writes) S.th[warp][row] = make_float2(a[0], b[0]);
+                    if (!kAnyZ || !active || !next_rows()) break;
+                    vb = 0;
+                    next_block();
+                    n_ent = row_ok ? (int)ent[0].x : 0, n_warp = (int)ent[0].y, i0 = 0;
+#pragma unroll
+                    for (int i = 0; i < VEC / 2; i++) t1[i] = t2[i] = 0ull;
                 }
             }
             __syncthreads();
@@ -783,12 +815,21 @@ __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L,
                         S.th[0][lane] = make_float2(th1, th2);
                         __syncwarp();
                         th1 = th2 = 0.0f;
-                        if (sl)
+                        if (!kAnyZ && sl) {
                             for (int r = 0; r < MZ; r++) {
                                 const float2 th = S.th[0][lane * MZ + r];
                                 th1 += th.x;
                                 th2 += th.y;
                             }
+                        } else if (sl) {  // the rows of the slice's block, or (one slice) of all blocks
+                            const int r0 = CZ == 1 ? 0 : first_row - rbase + lane * MZ;
+                            const int r1 = CZ == 1 ? min(32, end_row - rbase) : r0 + MZ;
+                            for (int r = r0; r < r1; r++) {
+                                const float2 th = S.th[0][r];
+                                th1 += th.x;
+                                th2 += th.y;
+                            }
+                        }
                     }
                     // even slices, then odd ones against the even ones' new values (the
                     // other lanes' results are dropped)
@@ -809,7 +850,7 @@ __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L,
                         if (has_p && lane < cz - 1) vp = up;
                     }
                     const float dx = skip ? 0.0f : cur - V;
-                    S.dx[lane] = MZ == 1 ? dx : __shfl_sync(0xffffffffu, dx, lane / MZ);
+                    S.dx[lane] = MZ == 1 || kAnyZ ? dx : __shfl_sync(0xffffffffu, dx, lane / MZ);  // kAnyZ: by slice
                     if (sl && !skip) {
                         x[col_off + sz] = cur;
                         if (kTile) cb[sz] = cur;
@@ -829,13 +870,12 @@ __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L,
 
             // ---- 4. apply e -= a dx ------------------------------------------------------
             {
-                Rows<VEC> dxv{};
-                if (row_ok) dxv = *reinterpret_cast<const Rows<VEC> *>(&S.dx[t0]);
-                bool any = false;
+                auto apply = [&](const Rows<VEC> &dxv) {
+                    bool any = false;
 #pragma unroll
-                for (int i = 0; i < VEC / 2; i++) any |= (dxv.p[i] & 0x7FFFFFFF7FFFFFFFull) != 0;
-                any = __any_sync(0xffffffffu, any);
-                if (any) {
+                    for (int i = 0; i < VEC / 2; i++) any |= (dxv.p[i] & 0x7FFFFFFF7FFFFFFFull) != 0;
+                    any = __any_sync(0xffffffffu, any);
+                    if (!any) return;
                     for (vb = 0;;) {
                         if (!kStaged && L.block_views < nv) next_block();
                         const int n = row_ok ? (int)ent[0].x : 0, n_warp = (int)ent[0].y;
@@ -854,11 +894,20 @@ __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L,
                         vb += L.block_views;
                         if (kStaged || vb >= nv) break;
                     }
+                };
+                if constexpr (!kAnyZ) {
+                    Rows<VEC> dxv{};
+                    if (row_ok) dxv = *reinterpret_cast<const Rows<VEC> *>(&S.dx[t0]);
+                    apply(dxv);
+                } else {
+                    auto dx_of = [&](int r) { return r >= first_row && r < end_row ? S.dx[(r - first_row) / MZ] : 0.0f; };
+                    rb = rbase - 32;
+                    while (next_rows()) apply(Rows<VEC>{{pack2(dx_of(rb + t0), dx_of(rb + t0 + 1))}});
                 }
                 // the column's update magnitude: the sum over its slices of |dx| (by
                 // the last warp: warp 0's chain is the longest)
                 if (warp == W - 1) {
-                    float m = lane < cz * MZ && lane % MZ == 0 ? fabsf(S.dx[lane]) : 0.0f;
+                    float m = (kAnyZ ? lane < cz : lane < cz * MZ && lane % MZ == 0) ? fabsf(S.dx[lane]) : 0.0f;
                     for (int off = 16; off > 0; off >>= 1) m += __shfl_xor_sync(0xffffffffu, m, off);
                     if (lane == 0) {
                         float *mp = mag + (size_t)f * nxy + c;
@@ -901,7 +950,7 @@ __device__ __forceinline__ void drain_copies(IcdSmem &S)
 // batch of loads in flight needs; at 72 registers (seven CTAs) the spills cost
 // more than the occupancy gave (4-D workload, iteration with its NH passes: 16.1
 // against 12.0 ms).
-template <int VEC, bool kStaged, bool kTile, int kHuber, int kBatch>
+template <int VEC, bool kStaged, bool kTile, int kHuber, int kBatch, bool kAnyZ>
 __global__ void __launch_bounds__(kMaxWarps * 32, 2) icd_phase_kernel(
     Geom g, IcdLaunch L, IcdConst K, const uint32_t *__restrict__ table, const int32_t *__restrict__ view_first,
     const uint8_t *__restrict__ mask, float *__restrict__ x, float *__restrict__ err, const float *__restrict__ wgt,
@@ -935,8 +984,8 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 2) icd_phase_kernel(
             sy = KC * (rem / hx) + color / KC;
         }
         if (sx >= L.n_sv_x || sy >= L.n_sv_y) continue;  // uniform
-        icd_update_sv<VEC, kStaged, kTile, kHuber, kBatch>(g, L, K, table, view_first, mask, x, err, wgt, mag, f, sx, sy,
-                                                          S, cnt, s_dyn);
+        icd_update_sv<VEC, kStaged, kTile, kHuber, kBatch, kAnyZ>(g, L, K, table, view_first, mask, x, err, wgt, mag, f,
+                                                                  sx, sy, S, cnt, s_dyn);
     }
     drain_copies(S);
     flush_counts(cnt, stats);
@@ -979,14 +1028,14 @@ static IcdMode icd_plan_shared(const Geom &g, IcdLaunch &L, int vec, int batch, 
     return mode;
 }
 
-template <int VEC, bool kStaged, bool kTile, int kHuber, int kBatch>
+template <int VEC, bool kStaged, bool kTile, int kHuber, int kBatch, bool kAnyZ = false>
 static void launch_mode(const Geom &g, const IcdLaunch &L, const IcdConst &K, const uint32_t *d_table,
                         const int32_t *d_view_first, const uint8_t *d_mask, float *d_x, float *d_err,
                         const float *d_w, float *d_mag, IcdStats *d_stats, unsigned int *d_queue, cudaStream_t st)
 {
     const int threads = L.warps * 32;
     const size_t smem = (size_t)L.shared_bytes;
-    const auto kernel = icd_phase_kernel<VEC, kStaged, kTile, kHuber, kBatch>;
+    const auto kernel = icd_phase_kernel<VEC, kStaged, kTile, kHuber, kBatch, kAnyZ>;
     // resident CTAs per SM, cached per (device, block size, shared memory) so a
     // launch being captured into a CUDA graph makes no occupancy query
     struct Occ {
@@ -1038,6 +1087,18 @@ static void launch_vec(const Geom &g, const IcdLaunch &L_, const IcdConst &K, co
 #undef MBIR_MODE
 }
 
+// Columns of more than 32 rows whose slices' rows do not divide 32 (z scales that are no
+// power of two, or above 32): the lists come from global memory, two rows a lane.
+static void launch_any_z(const Geom &g, const IcdLaunch &L_, const IcdConst &K, const uint32_t *d_table,
+                         const int32_t *d_view_first, const uint8_t *d_mask, float *d_x, float *d_err, const float *d_w,
+                         float *d_mag, IcdStats *d_stats, unsigned int *d_queue, cudaStream_t st)
+{
+    IcdLaunch L = L_;
+    icd_plan_shared(g, L, 2, 8, ICD_PLAIN);
+    (K.huber ? launch_mode<2, false, false, 1, 8, true> : launch_mode<2, false, false, 0, 8, true>)(
+        g, L, K, d_table, d_view_first, d_mask, d_x, d_err, d_w, d_mag, d_stats, d_queue, st);
+}
+
 IcdConst make_icd_const(const Geom &g)
 {
     IcdConst K;
@@ -1069,6 +1130,10 @@ void launch_icd_phase(const Geom &g, const IcdLaunch &L, const uint32_t *d_table
                       IcdStats *d_stats, unsigned int *d_queue, cudaStream_t st)
 {
     const IcdConst K = make_icd_const(g);
+    if (g.N_t > 32 && 32 % g.z_overlap) {
+        launch_any_z(g, L, K, d_table, d_view_first, d_mask, d_x, d_err, d_w, d_mag, d_stats, d_queue, st);
+        return;
+    }
     const bool v4 = g.N_t % 4 == 0;
     // entries in flight: 8, or 4 where no view group has more (one view each: a
     // batch is then mostly filling), or as the caller asks
