@@ -51,6 +51,7 @@ namespace {
 
 constexpr int kMaxWarps = 8;
 constexpr int kMaxSvCols = 256;  // sv <= 16
+constexpr float kMinNormal = 1.17549435e-38f;  // 2^-126
 
 __device__ __forceinline__ uint64_t mix64(uint64_t z)
 {
@@ -87,7 +88,8 @@ __device__ __forceinline__ float rcp_hw(float x)
 }
 // N weights times their filter coefficients f (which carry the 1 / sq), side by
 // side and without branches, so that the N chains of about 130 cycles run in
-// each other's shadow. isqp = 1 / sqp; at d = 0 the weight is q / (sq c).
+// each other's shadow. isqp = 1 / sqp; at d = 0 the weight is q / (sq c), and below
+// 2^-126, which the logarithm takes for zero (an infinite |d|^(q-2) at q < 2), too.
 template <int N>
 __device__ __forceinline__ void qg_coef(const float (&d)[N], const float (&f)[N], float q, float qmp, float isqp,
                                         float c, float qoc, float (&cf)[N])
@@ -106,7 +108,7 @@ __device__ __forceinline__ void qg_coef(const float (&d)[N], const float (&f)[N]
         for (int i = 0; i < N; i++) cf[i] *= ex2_hw((q - 2.0f) * l[i]);
     }
 #pragma unroll
-    for (int i = 0; i < N; i++) cf[i] = f[i] * (d[i] == 0.0f ? qoc : cf[i]);
+    for (int i = 0; i < N; i++) cf[i] = f[i] * (fabsf(d[i]) < kMinNormal ? qoc : cf[i]);
 }
 
 // The one arrival of a copy's mbarrier phase, and the bytes the phase waits for.

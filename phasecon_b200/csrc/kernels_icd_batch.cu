@@ -18,6 +18,7 @@ namespace {
 
 constexpr int kMaxWarps = 8;
 constexpr int kMaxSvCols = 256;  // sv <= 16
+constexpr float kMinNormal = 1.17549435e-38f;  // 2^-126
 
 __device__ __forceinline__ uint64_t mix64(uint64_t z)
 {
@@ -34,7 +35,8 @@ __device__ __forceinline__ uint64_t mix64(uint64_t z)
 // evaluated ~28 times per voxel update, so it uses the hardware base-2
 // logarithm / exponential (one logarithm for both powers) and reciprocal:
 // FP32 arithmetic whose rounding the FP64 MAP cost, by which the method's
-// result is measured, does not see.
+// result is measured, does not see. Differences below 2^-126 count as zero: the
+// logarithm takes them for it.
 __device__ __forceinline__ float lg2_hw(float x)
 {
     float r;
@@ -55,7 +57,7 @@ __device__ __forceinline__ float rcp_hw(float x)
 }
 __device__ __forceinline__ float qg_weight(float d, float q, float qmp, float isq, float isqp, float c, float b0)
 {
-    if (d == 0.0f) return b0;
+    if (fabsf(d) < kMinNormal) return b0;
     const float l = lg2_hw(fabsf(d));
     const float t1 = ex2_hw(qmp * l) * isqp;
     const float rt3 = rcp_hw(c + t1);
