@@ -1006,12 +1006,14 @@ struct UNet {
     // = a stack of D / Df frames of Df slices each
     int D = 0, H = 0, W = 0, Df = 0;
     bool has_grads = false;
+    bool has_inputs = false;  // every decoder input written out, in up and cat
     std::vector<std::pair<void *, size_t>> bufs;     // activation blocks in use (pointer, bytes)
     std::multimap<size_t, void *> spare;              // released blocks kept for reuse, by size
     bf16 *x0 = nullptr;
     bf16 *act[4][2] = {};  // encoder level l: conv a, conv b (= skip)
     bf16 *pool[3] = {};    // pooled encoder output of level l (input of level l+1)
-    bf16 *up[3] = {}, *u[3] = {}, *cat[3] = {}, *dec[3][2] = {};
+    bf16 *u[3] = {}, *dec[3][2] = {};
+    bf16 *up[3] = {}, *cat[3] = {};  // upsampled and concatenated inputs, where they are not read in place
     bf16 *gact[4][2] = {}, *gpool[3] = {}, *gup[3] = {}, *gu[3] = {}, *gcat[3] = {}, *gdec[3][2] = {};
     float *out = nullptr;
     double *d_loss = nullptr;
@@ -1032,13 +1034,15 @@ struct UNet {
         for (auto &b : bufs) spare.emplace(b.second, b.first);
         bufs.clear();
         D = H = W = Df = 0;
-        has_grads = false;
+        has_grads = has_inputs = false;
     }
     int init(int base, uint64_t seed);
     int ensure(int d, int h, int w, int frames = 1, bool grads = true);
     long long vox(int l) const { return (long long)(D >> l) * (H >> l) * (W >> l); }
     void conv(int i, const ConvIn &in, bf16 *o, int l, bool relu);
     void conv_tiles(int i, bool grad, const ConvIn &in, int Kin, const float *bias, bf16 *o, int Nout, int l, bool relu);
+    // the first of decoder level l's three convolutions (after the upsampling)
+    static int decoder_conv(int l) { return 8 + 3 * (2 - l); }
     // whether convolution i at level l reads a concatenated or upsampled input in
     // place (else it is written out first)
     bool in_place(int i, int l) const
@@ -1134,7 +1138,7 @@ int UNet::init(int base, uint64_t seed)
 
 int UNet::ensure(int d, int h, int w, int frames, bool grads)
 {
-    if (d * frames == D && d == Df && h == H && w == W && (has_grads || !grads)) return 0;
+    if (d * frames == D && d == Df && h == H && w == W && (has_grads || !grads) && (has_inputs || tensor_path)) return 0;
     if (d % 8 || h % 8 || w % 8 || d < 8 || h < 8 || w < 8)
         return fail("U-Net grid sizes must be multiples of 8 (got %d x %d x %d)", d, h, w);
     if (frames > 1 && d % 16)
@@ -1145,6 +1149,7 @@ int UNet::ensure(int d, int h, int w, int frames, bool grads)
     H = h;
     W = w;
     has_grads = grads;
+    has_inputs = !tensor_path;
     const int C[4] = {c, 2 * c, 4 * c, 8 * c};
     cudaError_t e = cudaSuccess;
     auto block = [&](void **p, size_t bytes) {
@@ -1173,11 +1178,13 @@ int UNet::ensure(int d, int h, int w, int frames, bool grads)
     for (int l = 0; l < 3; l++) {
         alloc(&pool[l], vox(l + 1) * C[l]);
         galloc(&gpool[l], vox(l + 1) * C[l]);
-        alloc(&up[l], vox(l) * C[l + 1]);
+        const int iu = decoder_conv(l);
+        up[l] = cat[l] = nullptr;
+        if (!in_place(iu, l)) alloc(&up[l], vox(l) * C[l + 1]);
         galloc(&gup[l], vox(l) * C[l + 1]);
         alloc(&u[l], vox(l) * C[l]);
         galloc(&gu[l], vox(l) * C[l]);
-        alloc(&cat[l], vox(l) * 2 * C[l]);
+        if (!in_place(iu + 1, l)) alloc(&cat[l], vox(l) * 2 * C[l]);
         galloc(&gcat[l], vox(l) * 2 * C[l]);
         for (int k = 0; k < 2; k++) {
             alloc(&dec[l][k], vox(l) * C[l]);
