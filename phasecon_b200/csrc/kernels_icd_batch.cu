@@ -66,29 +66,10 @@ __device__ __forceinline__ float qg_weight(float d, float q, float qmp, float is
     return r;
 }
 
-template <int KW>
-struct Rec {
-    uint4 w[KW];
-};
-
-template <int KW>
-__device__ __forceinline__ Rec<KW> load_rec(const uint32_t *p)
+// A record: header and three values (a batch's problems have voxel scale 1).
+__device__ __forceinline__ float rec_val(const uint4 &r, int q)
 {
-    Rec<KW> r;
-    const uint4 *q = reinterpret_cast<const uint4 *>(p);
-#pragma unroll
-    for (int i = 0; i < KW; i++) r.w[i] = __ldg(q + i);
-    return r;
-}
-
-template <int KW>
-__device__ __forceinline__ float rec_val(const Rec<KW> &r, int q)
-{
-    // word 1 + q of the record
-    const int wi = 1 + q;
-    const uint4 &u = r.w[wi >> 2];
-    const uint32_t bits = (wi & 3) == 0 ? u.x : (wi & 3) == 1 ? u.y : (wi & 3) == 2 ? u.z : u.w;
-    return __uint_as_float(bits);
+    return __uint_as_float(q == 0 ? r.y : q == 1 ? r.z : r.w);
 }
 
 template <int VEC>
@@ -154,33 +135,33 @@ __device__ __forceinline__ void flush_counts(IcdCount &cnt, IcdStats *stats)
 // sinogram row offset `row0` within each A entry's row, views gfirst,
 // gfirst + gstride, ... of the column): theta1 = -sum a w e,
 // theta2 = sum a^2 w with a = A value x delta_t (XT_VoxUpdate.c:56-85).
-template <int KW, int kUnroll, int VEC>
+template <int kUnroll, int VEC>
 __device__ __forceinline__ void theta_pass(const IcdConst &K, const uint32_t *col_rec, const float *__restrict__ err,
                                            const float *__restrict__ wgt, int gfirst, int gstride, int nv, int RW,
                                            int NT, int row0, float (&th1)[VEC], float (&th2)[VEC])
 {
     using VT = typename VecF<VEC>::T;
     for (int v0 = gfirst; v0 < nv; v0 += kUnroll * gstride) {
-        Rec<KW> R[kUnroll];
+        uint4 R[kUnroll];
 #pragma unroll
         for (int u = 0; u < kUnroll; u++) {
             const int v = v0 + u * gstride;
-            if (v < nv) R[u] = load_rec<KW>(col_rec + (size_t)v * RW);
-            else R[u].w[0].x = 0u;
+            if (v < nv) R[u] = __ldg(reinterpret_cast<const uint4 *>(col_rec + (size_t)v * RW));
+            else R[u].x = 0u;
         }
 #pragma unroll
         for (int u = 0; u < kUnroll; u++) {
-            const uint32_t hdr = R[u].w[0].x;
+            const uint32_t hdr = R[u].x;
             const int cnt_q = hdr >> 24;
             // sinogram rows stay below 2^24 and N_t rows each: 32-bit offsets
             const unsigned sb = (hdr & 0xFFFFFFu) * (unsigned)NT + (unsigned)row0;
 #pragma unroll
-            for (int q = 0; q < 4 * KW - 1; q++) {
+            for (int q = 0; q < 3; q++) {
                 if (q < cnt_q) {
                     float ev[VEC], wv[VEC];
                     VecF<VEC>::get(__ldcg(reinterpret_cast<const VT *>(err + (sb + (unsigned)(q * NT)))), ev);
                     VecF<VEC>::get(__ldg(reinterpret_cast<const VT *>(wgt + (sb + (unsigned)(q * NT)))), wv);
-                    const float a = rec_val<KW>(R[u], q) * K.dt;
+                    const float a = rec_val(R[u], q) * K.dt;
 #pragma unroll
                     for (int i = 0; i < VEC; i++) {
                         float ww = wv[i];
@@ -201,7 +182,7 @@ __device__ __forceinline__ void theta_pass(const IcdConst &K, const uint32_t *co
 // One column's theta: every lane's partial sums (theta_pass, when `run`),
 // folded over the view groups of the warp and stored by group 0 into the
 // warp's row of S.th1 / S.th2.
-template <int KW, int kUnroll, int VEC>
+template <int kUnroll, int VEC>
 __device__ __forceinline__ void theta_column(const IcdConst &K, const uint32_t *col_rec, const float *__restrict__ err,
                                              const float *__restrict__ wgt, int gfirst, int gstride, int nv, int RW,
                                              int NT, int row0, bool run, int lprp, int grp, int t0, int warp,
@@ -210,7 +191,7 @@ __device__ __forceinline__ void theta_column(const IcdConst &K, const uint32_t *
     float th1[VEC], th2[VEC];
 #pragma unroll
     for (int i = 0; i < VEC; i++) th1[i] = th2[i] = 0.0f;
-    if (run) theta_pass<KW, kUnroll, VEC>(K, col_rec, err, wgt, gfirst, gstride, nv, RW, NT, row0, th1, th2);
+    if (run) theta_pass<kUnroll, VEC>(K, col_rec, err, wgt, gfirst, gstride, nv, RW, NT, row0, th1, th2);
     for (int off = lprp; off < 32; off <<= 1) {
 #pragma unroll
         for (int i = 0; i < VEC; i++) {
@@ -230,12 +211,11 @@ __device__ __forceinline__ void theta_column(const IcdConst &K, const uint32_t *
 // Update the voxel columns of super-voxel (sx, sy) of frame f; the whole CTA
 // cooperates (the four passes of a column are those of the one-problem sweep: neighbourhood,
 // theta, solve, apply).
-// KW: 16-byte words per A record (1, 2, 3 for voxel scale 1, 2, 4);
 // kUnroll: views whose records and sinogram entries are in flight together;
 // VEC: consecutive detector rows one lane owns (4 when N_t % 4 == 0, else 2);
 // The data term (quadratic or generalised Huber, XT_VoxUpdate.c:68-82) is decided per
 // problem at run time (K.huber).
-template <int KW, int kUnroll, int VEC>
+template <int kUnroll, int VEC>
 __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L, const IcdConst &K,
                                               const uint32_t *__restrict__ table,
                                               const int32_t *__restrict__ view_first,
@@ -378,11 +358,9 @@ __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L,
             //         waiting for the other warps; otherwise after it, and only
             //         for an active column -------------------------------------------
             const bool sure = !L.zero_skipping || iter <= 1 || __any_sync(0xffffffffu, zl && V != 0.0f);
-            // a thread whose wait gave up reads no record (their headers address
-            // the sinogram); the CTA leaves after the barrier
             if (sure)
-                theta_column<KW, kUnroll, VEC>(K, col_rec, err, wgt, gfirst, gstride, nv, RW, NT,
-                                                               rbase + t0, row_ok, lprp, grp, t0, warp, S);
+                theta_column<kUnroll, VEC>(K, col_rec, err, wgt, gfirst, gstride, nv, RW, NT, rbase + t0, row_ok, lprp, grp,
+                                           t0, warp, S);
             const int any_active = __syncthreads_or(active_pred);
             if (!any_active) {
                 if (warp == 0 && zl) cnt.skip++;
@@ -390,8 +368,8 @@ __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L,
                 continue;  // uniform across the CTA
             }
             if (!sure) {  // uniform across the CTA
-                theta_column<KW, kUnroll, VEC>(K, col_rec, err, wgt, gfirst, gstride, nv, RW, NT,
-                                                               rbase + t0, row_ok, lprp, grp, t0, warp, S);
+                theta_column<kUnroll, VEC>(K, col_rec, err, wgt, gfirst, gstride, nv, RW, NT, rbase + t0, row_ok, lprp, grp,
+                                           t0, warp, S);
                 __syncthreads();
             }
 
@@ -488,22 +466,22 @@ __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L,
                 }
                 if (any) {
                     for (int v0 = gfirst; v0 < nv; v0 += kUnroll * gstride) {
-                        Rec<KW> R[kUnroll];
+                        uint4 R[kUnroll];
 #pragma unroll
                         for (int u = 0; u < kUnroll; u++) {
                             const int v = v0 + u * gstride;
-                            if (v < nv) R[u] = load_rec<KW>(col_rec + (size_t)v * RW);
-                            else R[u].w[0].x = 0u;
+                            if (v < nv) R[u] = __ldg(reinterpret_cast<const uint4 *>(col_rec + (size_t)v * RW));
+                            else R[u].x = 0u;
                         }
 #pragma unroll
                         for (int u = 0; u < kUnroll; u++) {
-                            const uint32_t hdr = R[u].w[0].x;
+                            const uint32_t hdr = R[u].x;
                             const int cnt_q = hdr >> 24;
                             const unsigned sb = (hdr & 0xFFFFFFu) * (unsigned)NT + (unsigned)(rbase + t0);
 #pragma unroll
-                            for (int q = 0; q < 4 * KW - 1; q++) {
+                            for (int q = 0; q < 3; q++) {
                                 if (q < cnt_q) {
-                                    const float a = -(rec_val<KW>(R[u], q) * K.dt);
+                                    const float a = -(rec_val(R[u], q) * K.dt);
                                     float d[VEC];
 #pragma unroll
                                     for (int i = 0; i < VEC; i++) d[i] = a * dxv[i];
@@ -527,9 +505,8 @@ __device__ __forceinline__ void icd_update_sv(const Geom &g, const IcdLaunch &L,
 // its item), so the CTAs working at any moment spread over the problems; a
 // CTA keeps the descriptor of its current problem in shared memory and
 // reloads it when its next item belongs to another problem. Problems of one
-// launch share the record width and the detector-row vector width (template
-// parameters).
-template <int KW, int kUnroll, int VEC>
+// launch share the detector-row vector width (a template parameter).
+template <int kUnroll, int VEC>
 __global__ void __launch_bounds__(kMaxWarps * 32, 4) icd_batch_kernel(const BatchDesc *__restrict__ descs,
                                                                       const int2 *__restrict__ item_map, int total,
                                                                       int phase, unsigned int *__restrict__ queue)
@@ -563,8 +540,8 @@ __global__ void __launch_bounds__(kMaxWarps * 32, 4) icd_batch_kernel(const Batc
         const int sx = K * (rem % hx) + color % K;
         const int sy = K * (rem / hx) + color / K;
         if (sx >= P.L.n_sv_x || sy >= P.L.n_sv_y) continue;
-        icd_update_sv<KW, kUnroll, VEC>(P.g, P.L, P.K, P.table, P.view_first, P.mask, P.x, P.err, P.w, P.mag,
-                                               f, sx, sy, S, cnt);
+        icd_update_sv<kUnroll, VEC>(P.g, P.L, P.K, P.table, P.view_first, P.mask, P.x, P.err, P.w, P.mag, f, sx, sy, S,
+                                    cnt);
     }
     if (cur >= 0) flush_counts(cnt, P.stats);
 }
@@ -598,16 +575,16 @@ int batch_grid(int vec, int warps)
     int dev = 0, sms = 148, per_sm = 1;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    if (vec == 4) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, icd_batch_kernel<1, 2, 4>, warps * 32, 0);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, icd_batch_kernel<1, 2, 2>, warps * 32, 0);
+    if (vec == 4) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, icd_batch_kernel<2, 4>, warps * 32, 0);
+    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, icd_batch_kernel<2, 2>, warps * 32, 0);
     return sms * (per_sm > 0 ? per_sm : 1);
 }
 
 void launch_icd_batch(int vec, int warps, int grid, const BatchDesc *d_descs, const int2 *d_item_map, int total,
                       int phase, unsigned int *d_queue, cudaStream_t st)
 {
-    if (vec == 4) icd_batch_kernel<1, 2, 4><<<grid, warps * 32, 0, st>>>(d_descs, d_item_map, total, phase, d_queue);
-    else icd_batch_kernel<1, 2, 2><<<grid, warps * 32, 0, st>>>(d_descs, d_item_map, total, phase, d_queue);
+    if (vec == 4) icd_batch_kernel<2, 4><<<grid, warps * 32, 0, st>>>(d_descs, d_item_map, total, phase, d_queue);
+    else icd_batch_kernel<2, 2><<<grid, warps * 32, 0, st>>>(d_descs, d_item_map, total, phase, d_queue);
 }
 
 void launch_batch_begin(BatchDesc *d_descs, int n, cudaStream_t st)
