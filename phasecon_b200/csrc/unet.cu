@@ -755,10 +755,9 @@ __global__ void maxpool_kernel(const bf16 *__restrict__ in, int C, int D, int H,
     }
 }
 
-// the gradient goes to the first input of each 2x2x2 block that holds the max
+// gin += the gradient at the first input of each 2x2x2 block that holds the max
 __global__ void maxpool_grad_kernel(const bf16 *__restrict__ in, const bf16 *__restrict__ out,
-                                    const bf16 *__restrict__ gout, int C, int D, int H, int W, bf16 *__restrict__ gin,
-                                    int accumulate)
+                                    const bf16 *__restrict__ gout, int C, int D, int H, int W, bf16 *__restrict__ gin)
 {
     const int d = D / 2, h = H / 2, w = W / 2;
     const long long n = (long long)d * h * w * C;
@@ -773,7 +772,7 @@ __global__ void maxpool_grad_kernel(const bf16 *__restrict__ in, const bf16 *__r
             const bool hit = !done && __bfloat162float(in[vi * C + c]) == m;
             done |= hit;
             const float add = hit ? gv : 0.0f;
-            gin[vi * C + c] = __float2bfloat16(accumulate ? __bfloat162float(gin[vi * C + c]) + add : add);
+            gin[vi * C + c] = __float2bfloat16(__bfloat162float(gin[vi * C + c]) + add);
         }
     }
 }
@@ -1266,10 +1265,7 @@ void UNet::conv_back(int i, const ConvIn &in, const bf16 *o, bf16 *go, bf16 *gin
                                                                                           d_g + k.b, d, h, w);
     } else {
         const unsigned gx = (unsigned)std::max(1, std::min(tiles, 4 * 148 / std::max(1, nci)));
-        if (k.cout > 32) {
-            dim3 grid(gx, (unsigned)nci, (unsigned)((k.cout + 63) / 64));
-            conv_wgrad_tile_kernel<64><<<grid, 256, 0, st>>>(in.a, k.cin, go, k.cout, d_g + k.w, d, h, w);
-        } else if (k.cout > 16) {
+        if (k.cout > 16) {  // 24 at base 12: wider layers of every base have counts that are multiples of 8
             conv_wgrad_tile_kernel<32><<<dim3(gx, nci, 1), 256, 0, st>>>(in.a, k.cin, go, k.cout, d_g + k.w, d, h, w);
         } else {
             conv_wgrad_tile_kernel<16><<<dim3(gx, nci, 1), 256, 0, st>>>(in.a, k.cin, go, k.cout, d_g + k.w, d, h, w);
@@ -1392,7 +1388,7 @@ int UNet::backward(const float *d_target, double *loss)
                 reinterpret_cast<uint4 *>(gact[l][1]));
         else if (l < 3)
             maxpool_grad_kernel<<<grid_for(vox(l + 1) * C[l]), 256, 0, st>>>(act[l][1], pool[l], gpool[l], C[l],
-                                                                             D >> l, H >> l, W >> l, gact[l][1], 1);
+                                                                             D >> l, H >> l, W >> l, gact[l][1]);
         conv_back(ib, plain(act[l][0], C[l]), act[l][1], gact[l][1], gact[l][0], l);
         bf16 *gx = l > 0 ? gpool[l - 1] : nullptr;
         conv_back(ia, plain(l > 0 ? pool[l - 1] : x0, convs[ia].cin), act[l][0], gact[l][0], gx, l);
