@@ -181,7 +181,9 @@ struct IcdConst {
     float issq, issqp, istq, istqp;  // reciprocals of the scale powers sigma^q, sigma^(q-p) (space, time)
     float qocs, qoct;                // q / c: the surrogate weight at a zero difference times sigma^q
     float bs0, bt0;                  // the same over sigma^q
-    float huber_T, huber_T2, huber_delta;  // T2: T^2 less a margin for rounding
+    float huber_T, huber_delta;
+    float huber_T2, huber_T2hi;      // T^2 less and plus a margin for rounding
+    float huber_a, huber_a2, huber_ha;  // a = T delta, a^2, 1 / (2 a)
     int huber;
 };
 IcdConst make_icd_const(const Geom &g);
