@@ -92,9 +92,25 @@ __global__ void __launch_bounds__(256) nh_scatter_kernel(int n_frames, int NY, i
 // > threshold; and, when svcount is given, the selected columns of every
 // super-voxel with a histogram per (phase, count). One launch: as eleven (filter,
 // four histogram / pick pairs, ...) a pass's selection took about 65 us, most of it
-// launches and one thread scanning 256 bins.
+// launches and one thread scanning 256 bins. Images beyond 65,536 columns are filtered by
+// a launch of their own first: 27 us for 512 x 512 columns, 69 for 1024 x 1024, 234 for
+// 2048 x 2048 (filtered by the eight SMs of the cluster 80, 294 and 1,102; as eleven
+// launches 72, 124 and 358).
 constexpr int kSelCtas = 8, kSelThreads = 1024;
 constexpr int kSelKeys = 8;  // keys a thread keeps in registers (images up to 256 x 256 entirely)
+
+// The filtered map of a larger image, by the whole GPU: eight SMs a frame take longer over
+// the filter than over the rest of the selection.
+__global__ void __launch_bounds__(256) nh_filter_kernel(int n_frames, int NY, int NX, const float *__restrict__ mag,
+                                                        float *__restrict__ filt)
+{
+    const int nxy = NX * NY;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < (long long)n_frames * nxy;
+         i += (long long)gridDim.x * blockDim.x) {
+        const int f = (int)(i / nxy), c = (int)(i - (long long)f * nxy);
+        filt[i] = vsc_filter(mag + (size_t)f * nxy, c / NX, c % NX, NY, NX);
+    }
+}
 
 __device__ __forceinline__ void cluster_sync()
 {
@@ -110,7 +126,7 @@ __device__ __forceinline__ unsigned remote_load(const unsigned *p, unsigned rank
 
 __global__ void __cluster_dims__(kSelCtas, 1, 1) __launch_bounds__(kSelThreads)
     nh_select_kernel(int NY, int NX, int k, const float *__restrict__ mag, const uint8_t *__restrict__ mask,
-                     float *__restrict__ filt, uint8_t *__restrict__ sel, int sv, int K, int *__restrict__ svcount,
+                     const float *__restrict__ filt, uint8_t *__restrict__ sel, int sv, int K, int *__restrict__ svcount,
                      int *__restrict__ hist_out)
 {
     __shared__ unsigned s_hist[256], s_sum[256];
@@ -118,16 +134,16 @@ __global__ void __cluster_dims__(kSelCtas, 1, 1) __launch_bounds__(kSelThreads)
     const int f = blockIdx.x / kSelCtas, rank = blockIdx.x % kSelCtas;
     const int nxy = NX * NY, first = rank * kSelThreads + threadIdx.x, stride = kSelCtas * kSelThreads;
     const float *m = mag + (size_t)f * nxy;
-    float *fm = filt + (size_t)f * nxy;
+    const float *fm = filt + (size_t)f * nxy;
     uint8_t *sm = sel + (size_t)f * nxy;
     unsigned key[kSelKeys];
-    const int rest = first + kSelKeys * stride;  // columns past those: filtered into fm, read back by the same thread
+    const int rest = first + kSelKeys * stride;  // columns past those: read from the map (nh_filter_kernel) each time
+    const bool mapped = nxy > kSelKeys * stride;
 #pragma unroll
     for (int i = 0; i < kSelKeys; i++) {
         const int c = first + i * stride;
-        key[i] = c < nxy ? __float_as_uint(vsc_filter(m, c / NX, c % NX, NY, NX)) : 0u;
+        key[i] = c >= nxy ? 0u : __float_as_uint(mapped ? fm[c] : vsc_filter(m, c / NX, c % NX, NY, NX));
     }
-    for (int c = rest; c < nxy; c += stride) fm[c] = vsc_filter(m, c / NX, c % NX, NY, NX);
     unsigned prefix = 0, pmask = 0, need = (unsigned)k + 1;
     bool found = true;
     for (int shift = 24; shift >= 0 && found; shift -= 8) {  // uniform over the cluster
@@ -139,6 +155,7 @@ __global__ void __cluster_dims__(kSelCtas, 1, 1) __launch_bounds__(kSelThreads)
 #pragma unroll
         for (int i = 0; i < kSelKeys; i++)
             if (first + i * stride < nxy) count(key[i]);
+#pragma unroll 8
         for (int c = rest; c < nxy; c += stride) count(__float_as_uint(fm[c]));
         cluster_sync();
         if (threadIdx.x < 256) {
@@ -183,6 +200,7 @@ __global__ void __cluster_dims__(kSelCtas, 1, 1) __launch_bounds__(kSelThreads)
         const int c = first + i * stride;
         if (c < nxy) sm[c] = (uint8_t)(k > 0 && mask[c] && (!found || key[i] > prefix));
     }
+#pragma unroll 8
     for (int c = rest; c < nxy; c += stride)
         sm[c] = (uint8_t)(k > 0 && mask[c] && (!found || __float_as_uint(fm[c]) > prefix));
     if (!svcount) return;
@@ -221,27 +239,40 @@ bool nh_items_supported(int n_frames, int N_y, int N_x, int sv)
     return n_frames <= 1024 && (N_x + sv - 1) / sv <= 2048 && (N_y + sv - 1) / sv <= 2048;
 }
 
-void launch_nh_select(int n_frames, int N_y, int N_x, const float *d_mag, const uint8_t *d_mask, int k,
-                      float *d_filt, uint8_t *d_sel, cudaStream_t st)
+// Returns the kernels launched.
+static int filter_large(int n_frames, int N_y, int N_x, const float *d_mag, float *d_filt, cudaStream_t st)
 {
-    nh_select_kernel<<<kSelCtas * n_frames, kSelThreads, 0, st>>>(N_y, N_x, k, d_mag, d_mask, d_filt, d_sel, 1, 1, nullptr,
-                                                                 nullptr);
+    const long long n = (long long)n_frames * N_y * N_x;
+    if ((long long)N_y * N_x <= (long long)kSelKeys * kSelCtas * kSelThreads) return 0;
+    nh_filter_kernel<<<(unsigned)std::min<long long>((n + 255) / 256, 148 * 8), 256, 0, st>>>(n_frames, N_y, N_x, d_mag, d_filt);
+    return 1;
 }
 
-void launch_nh_select_items(int n_frames, int N_y, int N_x, const float *d_mag, const uint8_t *d_mask, int k,
-                            float *d_filt, uint8_t *d_sel, int sv, int K, uint32_t *d_items, int *d_n_items,
-                            int *d_scratch, cudaStream_t st)
+int launch_nh_select(int n_frames, int N_y, int N_x, const float *d_mag, const uint8_t *d_mask, int k,
+                     float *d_filt, uint8_t *d_sel, cudaStream_t st)
+{
+    const int launched = filter_large(n_frames, N_y, N_x, d_mag, d_filt, st);
+    nh_select_kernel<<<kSelCtas * n_frames, kSelThreads, 0, st>>>(N_y, N_x, k, d_mag, d_mask, d_filt, d_sel, 1, 1, nullptr,
+                                                                 nullptr);
+    return launched + 1;
+}
+
+int launch_nh_select_items(int n_frames, int N_y, int N_x, const float *d_mag, const uint8_t *d_mask, int k,
+                           float *d_filt, uint8_t *d_sel, int sv, int K, uint32_t *d_items, int *d_n_items, int *d_scratch,
+                           cudaStream_t st)
 {
     const int nsx = (N_x + sv - 1) / sv, nsy = (N_y + sv - 1) / sv, maxc = sv * sv, KK = K * K;
     const size_t nsv = (size_t)n_frames * nsx * nsy, hsz = (size_t)KK * (maxc + 1);
     int *svcount = d_scratch, *hist = d_scratch + nsv, *cursor = hist + hsz;
     cudaMemsetAsync(hist, 0, 2 * hsz * sizeof(int), st);
+    const int launched = filter_large(n_frames, N_y, N_x, d_mag, d_filt, st);
     nh_select_kernel<<<kSelCtas * n_frames, kSelThreads, 0, st>>>(N_y, N_x, k, d_mag, d_mask, d_filt, d_sel, sv, K, svcount,
                                                                  hist);
     const int per_phase = nh_items_per_phase(n_frames, N_y, N_x, sv, K);
     nh_scatter_kernel<<<dim3((per_phase + 255) / 256, KK), 256, 0, st>>>(
         n_frames, N_y, N_x, sv, K, spread_multiplier(sv_slots(N_x, N_y, sv, K)), per_phase, svcount, hist, cursor, d_items,
         d_n_items);
+    return launched + 2;
 }
 
 }  // namespace mbirgpu

@@ -250,8 +250,8 @@ void launch_batch_end(BatchDesc *d_descs, int n, cudaStream_t st);
 // value, N = N_x N_y (RandomizedSelect's threshold), i.e. the k largest.
 constexpr int kMaxNhPasses = 16;
 constexpr int kNhicdIterations = 10;  // NHICD_Iterations, XT_Init.c:406
-void launch_nh_select(int n_frames, int N_y, int N_x, const float *d_mag, const uint8_t *d_mask, int k,
-                      float *d_filt, uint8_t *d_sel, cudaStream_t st);
+int launch_nh_select(int n_frames, int N_y, int N_x, const float *d_mag, const uint8_t *d_mask, int k,
+                     float *d_filt, uint8_t *d_sel, cudaStream_t st);
 // Work lists of the non-homogeneous passes: for each of the K x K phases of
 // the (sv, K) tiling (phase p of frame f updates colour (p + f) mod K^2), the
 // super-voxels holding selected columns, ordered by their number of selected
@@ -262,8 +262,8 @@ int nh_items_per_phase(int n_frames, int N_y, int N_x, int sv, int K);
 size_t nh_items_scratch_ints(int n_frames, int N_y, int N_x, int sv, int K);
 bool nh_items_supported(int n_frames, int N_y, int N_x, int sv);
 // The selection (as launch_nh_select) and the work lists of a pass.
-void launch_nh_select_items(int n_frames, int N_y, int N_x, const float *d_mag, const uint8_t *d_mask, int k,
-                            float *d_filt, uint8_t *d_sel, int sv, int K, uint32_t *d_items, int *d_n_items,
-                            int *d_scratch, cudaStream_t st);
+int launch_nh_select_items(int n_frames, int N_y, int N_x, const float *d_mag, const uint8_t *d_mask, int k,
+                           float *d_filt, uint8_t *d_sel, int sv, int K, uint32_t *d_items, int *d_n_items,
+                           int *d_scratch, cudaStream_t st);
 
 }  // namespace mbirgpu

@@ -445,10 +445,10 @@ int Session::enqueue_iteration(int iter, bool graph_mode, int *launches_out)
                            (size_t)nh_phases * per_phase <= nh_items_cap &&
                            nh_items_scratch_ints(g.N_time, g.N_y, g.N_x, nh_sv, nh_colors) <= nh_scratch_cap;
         if (lists)
-            launch_nh_select_items(g.N_time, g.N_y, g.N_x, d_mag, d_mask, k, d_filt, d_sel, nh_sv, nh_colors, d_nh_items,
-                                   d_nh_n, d_nh_scratch, st);
+            launches += launch_nh_select_items(g.N_time, g.N_y, g.N_x, d_mag, d_mask, k, d_filt, d_sel, nh_sv, nh_colors,
+                                               d_nh_items, d_nh_n, d_nh_scratch, st);
         else
-            launch_nh_select(g.N_time, g.N_y, g.N_x, d_mag, d_mask, k, d_filt, d_sel, st);
+            launches += launch_nh_select(g.N_time, g.N_y, g.N_x, d_mag, d_mask, k, d_filt, d_sel, st);
         for (int ph = 0; ph < nh_phases; ph++) {
             Ln.phase = ph;
             Ln.items = lists ? d_nh_items + (size_t)ph * per_phase : nullptr;
@@ -457,7 +457,7 @@ int Session::enqueue_iteration(int iter, bool graph_mode, int *launches_out)
                              d_queue + kMaxPhases * (pass + 1) + ph, st);
         }
         if (rings && update_offset()) return -1;
-        launches += nh_phases + 1 + (lists ? 1 : 0);  // the selection, the work lists
+        launches += nh_phases;
     }
     if (nh > 0 && timing) CK(record(ev_pairs[1].second));
     CK(cudaGetLastError());
