@@ -432,10 +432,7 @@ __host__ __device__ inline int icd_list_cap(int views_per_group, int kmax, int b
     return (1 + (views_per_group * kmax + batch - 1) / batch * batch) | 1;
 }
 
-// Unpack the records of view group `group` (views group, group + gstride, ...
-// from v_begin below v_end) into `list`; called by all lanes of a warp, lane tq of
-// the group's lprp lanes taking every lprp-th of its views.
-// where i < n
+// one entry, where i < n
 __device__ __forceinline__ void put_entry(uint2 *p, unsigned off, float na, int i, int n)
 {
     asm volatile("{\n\t.reg .pred P;\n\tsetp.lt.s32 P, %3, %4;\n\t@P st.shared.v2.b32 [%0], {%1, %2};\n\t}" ::"r"(
@@ -444,6 +441,9 @@ __device__ __forceinline__ void put_entry(uint2 *p, unsigned off, float na, int 
                  : "memory");
 }
 
+// Unpack the records of view group `group` (views group, group + gstride, ...
+// from v_begin below v_end) into `list`; called by all lanes of a warp, lane tq of
+// the group's lprp lanes taking every lprp-th of its views.
 template <int kBatch>
 __device__ __forceinline__ void unpack_records(const uint32_t *rec, int RW, int NT, float dt, uint2 *list, int group,
                                                int gstride, int v_begin, int v_end, int tq, int lprp)

@@ -73,7 +73,7 @@ void launch_zfast_to_vol(const float *in, float *out, int N_time, int N_z, int N
 // shared memory by all lanes, as are the voxels.
 //
 // What bounds it: shared-memory wavefronts (4 a record: its voxels, its weights) and
-// issue (23 instructions a record), 68 % and 61 % busy; 16 B of table a record come
+// issue (23 instructions a record), 72 % and 64 % busy; 16 B of table a record come
 // from HBM. 256 x 256 x 32 x 8 voxels, 1024 views: 2.13 ms (the
 // table's 1.07 GB alone would take 0.16); with the band in shared memory instead of registers (4
 // wavefronts more for each entry) and tiles of 32 columns (twice the reductions)
@@ -278,8 +278,8 @@ __device__ __forceinline__ void load_rows(float (&v)[VEC], const float *p, bool 
 // record costs each column a lane's share, and for one view the tile's entries fall
 // on a few channels, which stay in L1. Twelve products (four views' entries) are
 // summed in FP32, these sums in FP64. VEC 4 where the rows are a multiple of 4
-// (16-byte loads), else 2 (the row counts are even). What bounds it: the latency of
-// the rows' loads (L1, 76 % hits) at 24 warps an SM; 256 x 256 x 32 x 8 voxels, 1024
+// (16-byte loads), else 2 (the row counts are even). What bounds it: issue (59 % busy) and the
+// latency of the rows' loads (L1, 78 % hits) at 24 warps an SM; 256 x 256 x 32 x 8 voxels, 1024
 // views: 1.26 ms; a row a lane and a column a warp 2.79, four views of one column a
 // warp 2.12 (its rows don't stay in L1), two or four CTAs an SM 1.40 and 1.58, the
 // next records not loaded ahead 1.30.

@@ -141,7 +141,6 @@ struct IcdLaunch {
     int stage_words, list_cap, list_words, block_views, shared_bytes;
 };
 
-
 // SV slots of one colour per frame and the items (all frames) of one phase.
 inline int sv_slots(int N_x, int N_y, int sv, int K)
 {

@@ -86,8 +86,8 @@ constexpr int kPcDefaultNmsLanes = 4;
 constexpr int kPcDefaultNmsCtas = 4;
 
 // Launch geometry of the three-pass transform for V views of R x C (powers of
-// two): fills d's sizes and per-CTA tiles, the dynamic shared memory of the
-// row and column passes, and raises the kernels' shared-memory limits.
+// two): fills d's sizes and per-CTA tiles, and the dynamic shared memory of the
+// row and column passes.
 int pc_transform_dims(PcDims &d, int V, int R, int C, size_t *smem_rows, size_t *smem_cols, int fft_radix = 0);
 // the FFT stage radix used when none is asked for
 constexpr int kPcDefaultFftRadix = 16;

@@ -225,8 +225,11 @@ int Session::init(const mbirgpu_problem *pb, const mbirgpu_options *o, int mult_
 // more, else 4; where the SVs leave SMs
 // idle (small images: at most one SV per SM), the length of a column's chain is
 // all that counts: 4, or 8 when the column's entries give a lane of one warp more
-// than 64 (sweep of a 100 x 100 x 38 Huber problem, 75 views a frame: 4.2 ms
-// with 4 warps, 2.9 with 8; 64 x 64 x 8, 90 views, 13 entries: 0.52 both ways).
+// than 64 (sweep of a 100 x 100 x 38 Huber problem, 75 views a frame, 101 entries:
+// 2.5 ms with 4 warps, 1.8 with 8; 64 x 64 x 8, 90 views, 13 entries: 0.42 and 0.38;
+// 128 x 128 x 16, 180 views, 51 entries: 1.15 and 0.97, so the line may lie lower).
+// Between, 3.5 SVs per SM (256 x 256 x 32, 4 frames of 128 views, Huber): 10.5 ms with 2
+// warps, 7.0 with 4, 8.6 with 8.
 // Fields the user fixed are kept.
 constexpr long long kSms = 148;
 
@@ -268,10 +271,10 @@ void Session::choose_schedule()
 
 // Schedule of the non-homogeneous passes: the user's, else the full sweep's
 // super-voxels and colours, with 4 warps per column where the SVs in flight fill
-// the GPU (4-D workload: 12.1 ms per iteration with 4, 13.5 with 2, 14.6 with 8)
+// the GPU (4-D workload: 12.0 ms per iteration with 4, 13.3 with 2, 14.7 with 8)
 // and twice the sweep's, up to 8, where they do not (chains of column updates
 // inside the few super-voxels that hold many selected columns: 100 x 100 x 38
-// Huber problem, 10.1 ms with 8 against 12.6 with 4).
+// Huber problem, 6.0 ms with 8 against 7.5 with 4).
 void Session::sync_nh_schedule()
 {
     nh_sv = opt.nh_sv_size > 0 ? std::min(opt.nh_sv_size, 16) : sv;

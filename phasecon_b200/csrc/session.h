@@ -41,7 +41,7 @@ struct Session {
     static constexpr int kQueueCounters = kMaxPhases * (1 + kMaxNhPasses);
     float *d_filt = nullptr;          // NH-ICD filtered update magnitudes [N_time][N_y][N_x]
     uint8_t *d_sel = nullptr;         // NH-ICD selected columns [N_time][N_y][N_x]
-    uint32_t *d_nh_items = nullptr;   // NH-ICD work lists (launch_nh_items), per phase
+    uint32_t *d_nh_items = nullptr;   // NH-ICD work lists (launch_nh_select_items), per phase
     int *d_nh_n = nullptr;            // their lengths [kMaxPhases]
     int *d_nh_scratch = nullptr;
     size_t nh_items_cap = 0, nh_scratch_cap = 0;  // ints allocated
