@@ -623,10 +623,14 @@ int Session::amatrix(int32_t *first, int32_t *count, float *values)
 // A volume of scratch beside d_tmp: the FP64 accumulator, whose content no call needs
 // from another, where it is large enough (n_vox <= 2 n_sino floats: all but scans of few
 // views), else an allocation in *own, which the caller frees. Two allocations and
-// releases a call took longer than the projections of small scans.
+// releases a call took longer than the projections of small scans. Work that an
+// asynchronous call (refresh_error, set_object) left on another stream may still be in
+// the accumulator: after a change of stream it is waited for, once.
 int Session::volume_scratch(float **vol, float **own)
 {
     *own = nullptr;
+    if (stream_changed) CK(cudaDeviceSynchronize());
+    stream_changed = false;
     size_t acc = 0;
     if (n_vox > 2 * n_sino && dalloc(own, n_vox, &acc)) return -1;
     *vol = *own ? *own : reinterpret_cast<float *>(d_acc);
@@ -890,6 +894,7 @@ int mbirgpu_session_info_get(const mbirgpu_session *sp, mbirgpu_session_info *in
 int mbirgpu_session_set_stream(mbirgpu_session *sp, void *stream)
 {
     SESSION(sp);
+    if (s->st != (cudaStream_t)stream) s->stream_changed = true;
     s->st = (cudaStream_t)stream;
     return 0;
 }

@@ -16,6 +16,7 @@ struct Session {
     mbirgpu_options opt{};
     cudaStream_t st = nullptr;
     int device = 0;  // the CUDA device that was current when the session was created
+    bool stream_changed = false;  // since the accumulator was last known to be idle
     float convg_thresh = 0;
     size_t n_sino = 0, n_vox = 0, device_bytes = 0;
     int n_assigned = 0;  // views that belong to some frame
